@@ -406,11 +406,68 @@ __device__ __forceinline__ auto current_view(const FieldStretchT<M>& f, const Fi
     return r;
 }
 
+// 2^x and log2 x by the hardware approximations (ex2/lg2.approx.ftz.f32):
+// the fast step controller only needs the next step size to a few digits.
+__device__ __forceinline__ float ex2_approx(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float lg2_approx(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // x^y correctly rounded to float: the double-precision power narrowed once
 // (its error is far below half a float ulp except within ~2^-28 of a float
 // rounding boundary).  The exact kernels use it so that the step controller's
 // decisions do not depend on one library's powf rounding.
 __device__ __forceinline__ float pow_cr(float x, float y) { return (float)pow((double)x, (double)y); }
+
+// The exact step controller's power, (float)pow((double)x, (double)0.2f) of
+// x = (float)((double)q / 11.09), q = tol / err.  The double form, kept out
+// of line, costs ~100 operations of the FP64 pipe (two lanes per clock and
+// SM); the float form below replaces it wherever the rounding is certain.
+static __device__ __noinline__ float step_scale_double(float q) { return pow_cr((float)((double)q / 11.09), 0.2f); }
+
+// x: q times 1 / 11.09 held as two floats (the pair is within 2^-47 of the
+// quotient).  s = x^0.2f: 5 x 0.2f is 1 + 2^-26 exactly, so s^5 = x (1 +
+// 2^-26 ln x) to 2^-45; two Newton steps on s^5 from the hardware log2 / exp2
+// with the fifth power as a pair of floats, the last one kept apart from s as
+// its correction (the pair is within 2^-45 of the power).  round_f2 rounds
+// both; where it is not sure (one in 10^4), and for x outside
+// [2^-20, 2^20] (a step grown 16 times, or cut far below rejection), the
+// double form decides.
+__device__ __forceinline__ float step_scale_exact(float q) {
+    constexpr double r = 1.0 / 11.09;
+    constexpr float rh = (float)r, rl = (float)(r - (double)(float)r);
+    bool sure = (q >= 0x1p-16f) & (q <= 0x1p+23f);
+    F2 xq;
+    xq.h = q * rh;
+    xq.l = __fmaf_rn(q, rl, __fmaf_rn(q, rh, -xq.h));
+    const float x = round_f2(xq, sure);
+    const float l2 = lg2_approx(x);
+    const float xc = x * (l2 * (float)(0.6931471805599453 * 0x1p-26));
+    float ri;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(x));
+    ri = 0.2f * ri;
+    F2 s = {ex2_approx(0.2f * l2), 0.f};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        s.h = s.h + s.l;
+        const float s2 = s.h * s.h, s2l = __fmaf_rn(s.h, s.h, -s2);
+        const float s4 = s2 * s2, s4l = __fmaf_rn(2.f * s2, s2l, __fmaf_rn(s2, s2, -s4));
+        const float s5 = s4 * s.h, s5l = __fmaf_rn(s4l, s.h, __fmaf_rn(s4, s.h, -s5));
+        s.l = s.h * (((x - s5) + (xc - s5l)) * ri);
+    }
+    const float y = round_f2(s, sure);
+    return sure ? y : step_scale_double(q);
+}
+
+// The smallest float not below 0.618: a float is below it exactly when its
+// double is below 0.618.
+constexpr float kAcceptScale = (double)0.618f >= 0.618 ? 0.618f : 0.618f + 0x1p-24f;
 
 // J.B / |B|^2, the twist integrand.  The fast form fixes its rounding
 // sequence with explicit multiply-adds: left as plain expressions, the
@@ -499,19 +556,6 @@ __device__ __forceinline__ void lane_begin(const F& f, const TraceJob<F>& J, Lan
     }
 }
 
-// 2^x and log2 x by the hardware approximations (ex2/lg2.approx.ftz.f32):
-// the fast step controller only needs the next step size to a few digits.
-__device__ __forceinline__ float ex2_approx(float x) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float lg2_approx(float x) {
-    float r;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
 // a - b on the packed f32x2 pipe
 __device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
     float2 d;
@@ -557,8 +601,8 @@ __device__ __forceinline__ int lane_control(const TraceJob<F>& J, Lane<EXACT>& L
     const qsl_trace_params& pr = J.prm;
     float scale;
     if (EXACT) {
-        scale = pow_cr((float)((double)(L.tol / err) / 11.09), 0.2f);
-        if ((double)scale < 0.618) {
+        scale = step_scale_exact(L.tol / err);
+        if (scale < kAcceptScale) {
             L.h = (float)((double)L.h * pr.reject_factor);
             if (pr.max_rejects > 0 && ++L.rej >= pr.max_rejects) {
                 L.out = L.p;
@@ -584,13 +628,9 @@ __device__ __forceinline__ int lane_control(const TraceJob<F>& J, Lane<EXACT>& L
     }
     L.rej = 0;
     float h = L.h * scale;
-    if (EXACT) {
-        if ((double)h > pr.h_max) h = (float)pr.h_max;
-        if ((double)h < pr.h_min) h = (float)pr.h_min;
-    } else {
-        if (h > J.lim.h_max) h = J.lim.h_max;  // a NaN step stays NaN, as above
-        if (h < J.lim.h_min) h = J.lim.h_min;
-    }
+    // (the same clamps in float, see StepLimits)
+    if (h > J.lim.h_max) h = J.lim.h_max;  // a NaN step stays NaN
+    if (h < J.lim.h_min) h = J.lim.h_min;
     L.h = h;
     return 0;
 }
@@ -827,7 +867,16 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
     // warp-uniform chunk window [c_next, c_end) of the work queue
     long long c_next = 0, c_end = 0;
     bool q_empty = false;
-    const long long chunk = J.chunk > 0 ? J.chunk : 256;
+    // lines per refill: the caller's choice, else an even share per warp of
+    // the grid between one warp's width (a small launch then uses every warp:
+    // with 256 the 128 x 128 plane ran on 64 of 2432 warps) and 256 (the
+    // neighbouring seeds that keep a warp's gathers together)
+    long long chunk = J.chunk;
+    if (QUEUE && chunk <= 0) {
+        const long long warps = (long long)gridDim.x * (blockDim.x / 32);
+        chunk = ((n + warps - 1) / warps + 31) / 32 * 32;
+        chunk = chunk < 32 ? 32 : (chunk > 256 ? 256 : chunk);
+    }
     long long next_static = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 
     while (true) {
