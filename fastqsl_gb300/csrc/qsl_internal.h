@@ -13,11 +13,22 @@ enum Layout { LAYOUT_SOA = 0, LAYOUT_F4 = 1, LAYOUT_H4B = 2, LAYOUT_H8C = 3 };
 constexpr int kStoreTypes = 4;
 enum Schedule { SCHED_QUEUE = 0, SCHED_STATIC = 1 };
 
-constexpr int kTraceBlock = 128;
+constexpr int kTraceBlock = kTraceThreads;
 
 // Blocks of `kernel` that fit on one SM at kTraceBlock threads, times the SM
 // count: the persistent grid.
 int persistent_grid(const void* kernel, int block, size_t smem = 0);
+
+// Grid of a static tracer launch of n lines, for a kernel of which
+// `resident` blocks fit on the GPU at a time: two warps per 32 lines, one per
+// direction (trace_lines' split), where all of them are resident together,
+// else one thread per line.
+inline int static_grid(long long n, int resident) {
+    const long long pairs = 64 * ((n + 31) / 32);
+    long long g = pairs <= (long long)resident * kTraceBlock ? pairs : n;
+    g = (g + kTraceBlock - 1) / kTraceBlock;
+    return (int)(g < 1 ? 1 : (g > (1 << 30) ? (1 << 30) : g));
+}
 
 // trace_exact.cu (compiled with -fmad=false)
 cudaError_t launch_trace_exact(const TraceJob<FieldSoA>& J, bool twist, Schedule sched, long long n_host,

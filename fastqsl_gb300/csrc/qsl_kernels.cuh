@@ -10,7 +10,7 @@ namespace qsl {
 // (1 = compiler's choice).  Higher values trade registers (possibly spills)
 // for resident warps; the autotuner measures and picks.
 template <bool TWIST, bool QUEUE, class F, int MINB>
-__global__ void __launch_bounds__(kTraceBlock, MINB) k_trace_fast(const TraceJob<F> J) {
+__global__ void __launch_bounds__(kTraceBlock, MINB) k_trace_fast(const __grid_constant__ TraceJob<F> J) {
     trace_kernel_body<false, TWIST, QUEUE>(J);
 }
 
@@ -22,19 +22,15 @@ static cudaError_t launch_fast_minb(const TraceJob<F>& J, bool twist, Schedule s
                                : (const void*)k_trace_fast<false, true, F, MINB>)
                       : (twist ? (const void*)k_trace_fast<true, false, F, MINB>
                                : (const void*)k_trace_fast<false, false, F, MINB>);
-    int grid;
-    if (q) {
-        grid = persistent_grid(k, kTraceBlock);
-    } else {
-        long long g = (n_host + kTraceBlock - 1) / kTraceBlock;
-        // a device-side count (n_host is only the capacity): two resident
-        // waves of blocks stride over the lines instead of a grid over the
-        // whole capacity whose surplus blocks would each start and exit
-        if (J.s.n_dev) {
-            const long long cap = 2LL * persistent_grid(k, kTraceBlock);
-            if (cap > 0 && g > cap) g = cap;
-        }
-        grid = (int)(g < 1 ? 1 : (g > (1 << 30) ? (1 << 30) : g));
+    int grid = persistent_grid(k, kTraceBlock);
+    if (!q) {
+        // a device-side count (n_host is only the capacity): at most two
+        // resident waves of blocks stride over the lines instead of a grid
+        // over the whole capacity whose surplus blocks would each start and
+        // exit
+        const int waves = 2 * grid;
+        grid = static_grid(n_host, grid);
+        if (J.s.n_dev && waves > 0 && grid > waves) grid = waves;
     }
     if (grid <= 0) return cudaErrorInvalidConfiguration;
     if (q) {
@@ -96,6 +92,21 @@ static void launch_batch_minb(int grid, const TraceJob<F>* jobs, const long long
     else k_trace_batch<false, F, MINB><<<grid, kTraceBlock, 0, st>>>(jobs, begin, njobs, samples, line_lo, line_hi);
 }
 
+template <class F, int MINB>
+static const void* batch_kernel_minb(bool twist) {
+    return twist ? (const void*)k_trace_batch<true, F, MINB> : (const void*)k_trace_batch<false, F, MINB>;
+}
+template <class F>
+static const void* batch_kernel(int occupancy, bool twist) {
+    switch (occupancy) {
+        case 6: return batch_kernel_minb<F, 6>(twist);
+        case 7: return batch_kernel_minb<F, 7>(twist);
+        case 9: return batch_kernel_minb<F, 9>(twist);
+        case 10: return batch_kernel_minb<F, 10>(twist);
+        default: return batch_kernel_minb<F, 8>(twist);
+    }
+}
+
 template <class F>
 static cudaError_t launch_batch(const TraceJob<F>* jobs, const long long* begin, int njobs, long long total,
                                 bool twist, unsigned long long* samples, int max_blocks, long long line_lo,
@@ -104,9 +115,10 @@ static cudaError_t launch_batch(const TraceJob<F>* jobs, const long long* begin,
     if (line_lo < 0) line_lo = 0;
     if (line_hi < 0 || line_hi > total) line_hi = total;
     if (line_lo >= line_hi) return cudaSuccess;
-    long long g = (line_hi - line_lo + kTraceBlock - 1) / kTraceBlock;
-    if (max_blocks > 0 && g > max_blocks) g = max_blocks;  // the grid-stride loop covers the rest
-    const int grid = (int)(g > (1 << 30) ? (1 << 30) : g);
+    const int resident = persistent_grid(batch_kernel<F>(occupancy, twist), kTraceBlock);
+    if (resident <= 0) return cudaErrorInvalidConfiguration;
+    int grid = static_grid(line_hi - line_lo, resident);
+    if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;  // the grid-stride loop covers the rest
     switch (occupancy) {
         case 6: launch_batch_minb<F, 6>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
         case 7: launch_batch_minb<F, 7>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;

@@ -4,18 +4,31 @@
 // 383-464): forward trace -> end footpoint, backward trace -> start footpoint,
 // B at both footpoints and at the seed, B_flag, line length, optional twist.
 //
-// Scheduling: a persistent grid (a multiple of the SM count) in which every
-// lane owns one line at a time and, the moment its line finishes, takes the
-// next one from a device work counter (one warp-aggregated atomic per refill).
-// Lines whose lengths differ by orders of magnitude (RKF45 near nulls and
-// separators) therefore never hold a warp's other lanes idle.  A static mode
-// (one line per thread, no counter) is the plain baseline.
+// Scheduling: a warp takes 32 lines (neighbouring seeds when the order is a
+// tile order) and traces them in lockstep, each lane forward and then
+// backward; the footpoints, the samples of B and the outputs follow once for
+// the whole warp (trace_lines).  Where the launch has two threads per line,
+// the directions go to a pair of warps instead.  Static: the warp's lines
+// follow from its index; queue: a persistent grid whose warps take chunks of
+// lines from a device counter, for device-side counts and for lines whose
+// lengths differ by orders of magnitude between warps.
+//
+// What it replaced: every lane taking its next line from the queue as its
+// own ended, and doing its line's end then and there.  A warp's lanes were
+// then at different points of the loop (9-13 of 32 active, instruction-fetch
+// stalls at 10-15 cycles per issue in the exact kernels) and their gathers
+// scattered.  Drop-in RKF45 on 201 x 203 x 4 seeds with twist 11.0 -> 4.0 ms,
+// map of 256 x 512 seeds 11.0 -> 6.6 ms, RK4 on 128 x 128 seeds 5.0 -> 3.2 ms;
+// fast kernels: 100 x 100 seeds in 64^3 0.366 -> 0.244 ms, a 258 x 258 x 32
+// slab of 512 x 512 x 256 22.5 -> 21.4 ms.
 #pragma once
 #include <type_traits>
 #include "qsl_field.cuh"
 #include "../../include/fastqsl_gb300.h"
 
 namespace qsl {
+
+constexpr int kTraceThreads = 128;  // threads per block of every tracer kernel
 
 constexpr double kRefPi = 3.14159265;  // the reference's M_PI (TraceBlineAdaptive.cu:10)
 // 1 / (4 pi) for the fast twist increment: one float product per step and a
@@ -81,7 +94,7 @@ struct TraceJob {
     unsigned long long* queue;    // work counter, zero at launch; null = static
     unsigned long long* samples;  // optional: total field samples
     const unsigned* order;        // optional: line k traces seed order[k] and writes its outputs there
-    int chunk;                    // lines a warp takes from the queue at a time (QUEUE)
+    int chunk;                    // lines a warp takes from the queue at a time (QUEUE; 0 = chosen from n)
     int occupancy;                // resident-block variant of the fast kernels (0 = default)
 };
 
@@ -198,67 +211,77 @@ __device__ __forceinline__ float3 step_rkf45_fast_rolled(const F& f, float3 p, f
     return f3(scal(h, sol));
 }
 
+// The exact Fehlberg step: k = h b per stage, every product and sum rounded on
+// its own in the reference's order (sums from the left; a stage's input is
+// p plus its whole sum).  The stages are rolled as above: each stage's k adds
+// its term to the sums still to come, which is that order.  (Unrolled, the
+// exact samples do not fit the instruction cache: drop-in planes 18-35 %
+// slower.)
+template <class F>
+__device__ __forceinline__ float3 step_rkf45_exact(const F& f, float3 p, float h, float& err, unsigned& ns) {
+    const float3 zero = v3(0.f, 0.f, 0.f);
+    float3 slot[5] = {zero, zero, zero, zero, zero};
+    float3 sol = zero, e = zero;
+#pragma unroll 1
+    for (int st = 0; st < 6; ++st) {
+        const float3 k = h * sample<true>(f, st > 0 ? p + slot[0] : p, true);
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const float3 t = kFehlbergTab.a[st][i] * k;
+            slot[i] = st > 0 ? (i < 4 ? slot[i + 1] + t : t) : t;
+        }
+        const float3 ts = kFehlbergTab.b[st] * k, te = kFehlbergTab.e[st] * k;
+        sol = st > 0 ? sol + ts : ts;
+        e = st > 0 ? e + te : te;
+    }
+    err = norm(e);
+    ns += 6;
+    return sol;
+}
+
 template <bool EXACT, class F>
 __device__ __forceinline__ float3 step_rkf45(const F& f, float3 p, float h, float& err, unsigned& ns,
                                             float3* b_raw = nullptr) {
-    if constexpr (!EXACT && RolledStages<F>::value) return step_rkf45_fast_rolled(f, p, h, err, ns, b_raw);
-    if (!EXACT) return step_rkf45_fast(f, p, h, err, ns, b_raw);
-    using C = Fehlberg;
-    const float3 k1 = h * sample<EXACT>(f, p, true);
-    const float3 k2 = h * sample<EXACT>(f, p + C::a21 * k1, true);
-    const float3 k3 = h * sample<EXACT>(f, p + (C::a31 * k1 + C::a32 * k2), true);
-    const float3 k4 = h * sample<EXACT>(f, p + ((C::a41 * k1 + C::a42 * k2) + C::a43 * k3), true);
-    const float3 k5 = h * sample<EXACT>(f, p + (((C::a51 * k1 + C::a52 * k2) + C::a53 * k3) + C::a54 * k4), true);
-    const float3 k6 =
-        h * sample<EXACT>(f, p + ((((C::a61 * k1 + C::a62 * k2) + C::a63 * k3) + C::a64 * k4) + C::a65 * k5), true);
-    const float3 e = (((C::e1 * k1 + C::e3 * k3) + C::e4 * k4) + C::e5 * k5) + C::e6 * k6;
-    err = norm(e);
-    ns += 6;
-    return (((C::b1 * k1 + C::b3 * k3) + C::b4 * k4) + C::b5 * k5) + C::b6 * k6;
+    if constexpr (EXACT) return step_rkf45_exact(f, p, h, err, ns);
+    else if constexpr (RolledStages<F>::value) return step_rkf45_fast_rolled(f, p, h, err, ns, b_raw);
+    else return step_rkf45_fast(f, p, h, err, ns, b_raw);
 }
 
 // Classic RK4 on b (RK4, TraceBlineAdaptive.cu:259-267); returns the
 // increment.  The 1/6 factor is formed as (1./6.)*h in double and narrowed.
 template <bool EXACT, class F>
 __device__ __forceinline__ float3 step_rk4(const F& f, float3 p, float h, unsigned& ns, float3* b_raw = nullptr) {
-    const float3 k1 = (!EXACT && b_raw) ? sample_unit_raw(f, p, *b_raw) : sample<EXACT>(f, p, true);
+    if constexpr (EXACT) {
+        // the stages rolled (one sample in the loop body): the same
+        // operations in the same order
+        float3 q = p, sum = v3(0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int st = 0; st < 4; ++st) {
+            const float3 k = sample<true>(f, q, true);
+            const float3 hk = h * k;
+            q = p + (st < 2 ? hk / 2.f : hk);
+            sum = st == 0 ? k : (st < 3 ? sum + 2.f * k : sum + k);
+        }
+        ns += 4;
+        return (float)(1.0 / 6.0 * (double)h) * sum;
+    }
+    const float3 k1 = b_raw ? sample_unit_raw(f, p, *b_raw) : sample<EXACT>(f, p, true);
     const float3 k2 = sample<EXACT>(f, p + (h * k1) / 2.f, true);
     const float3 k3 = sample<EXACT>(f, p + (h * k2) / 2.f, true);
     const float3 k4 = sample<EXACT>(f, p + h * k3, true);
     ns += 4;
-    const float c = EXACT ? (float)(1.0 / 6.0 * (double)h) : h * (1.f / 6.f);
-    return c * (((k1 + 2.f * k2) + 2.f * k3) + k4);
+    return h * (1.f / 6.f) * (((k1 + 2.f * k2) + 2.f * k3) + k4);
 }
 
 // RK4 in the face-normal coordinate, dx/dq = b / b_d over dq = h
-// (RK4_boundary, TraceBlineAdaptive.cu:286-307).  Out of line (it runs once
-// per line end); the store view is taken by value so that the caller's copy
-// never has its address taken.  4 field samples.
+// (RK4_boundary, TraceBlineAdaptive.cu:286-307), its four stages in a rolled
+// loop (it runs once per line end).  4 field samples.
 template <bool EXACT, class F>
-__device__ __noinline__ float3 step_rk4_normal(const F f, float3 p, float h, int d) {
-    float3 b = sample_outlined<EXACT>(f, p, true);
-    const float3 k1 = b / comp(b, d);
-    b = sample_outlined<EXACT>(f, p + (h * k1) / 2.f, true);
-    const float3 k2 = b / comp(b, d);
-    b = sample_outlined<EXACT>(f, p + (h * k2) / 2.f, true);
-    const float3 k3 = b / comp(b, d);
-    b = sample_outlined<EXACT>(f, p + h * k3, true);
-    const float3 k4 = b / comp(b, d);
-    const float c = EXACT ? (float)(1.0 / 6.0 * (double)h) : h * (1.f / 6.f);
-    return p + c * (((k1 + 2.f * k2) + 2.f * k3) + k4);
-}
-
-// The same boundary RK4 inlined, its four stages in a rolled loop, for the
-// stretched-grid stores: the out-of-line form takes the store view by value,
-// and for their large views (coordinate arrays, per-axis constants, search
-// tables) the caller then keeps a copy of the view in local memory, which
-// the hot loop reads too.  The same operations in the same order.
-template <bool EXACT, class F>
-__device__ __forceinline__ float3 step_rk4_normal_rolled(const F& f, float3 p, float h, int d) {
+__device__ __forceinline__ float3 step_rk4_normal(const F& f, float3 p, float h, int d) {
     float3 k1 = v3(0.f, 0.f, 0.f), k2 = k1, k3 = k1, k4 = k1, q = p;
 #pragma unroll 1
     for (int st = 0; st < 4; ++st) {
-        const float3 b = sample<EXACT>(f, q, true);
+        const float3 b = sample_outlined<EXACT>(f, q, true);
         const float3 k = b / comp(b, d);
         if (st == 0) {
             k1 = k;
@@ -498,10 +521,12 @@ struct Lane {
     int steps;     // accepted steps
     int rej;       // trial steps rejected in a row
     unsigned dsign;  // sign bit of the step: 0 forward, 0x80000000 backward
-    long long line;
-    float3 out;    // footpoint of this direction when finished
+    float3 out;    // footpoint of this direction when finished (the point past the face before lane_foot)
     int flag;      // reference flag; bits 8.. hold the qsl_line_status when finished
 };
+
+// Lane::flag of a direction that left the box, until lane_foot classifies it
+constexpr int kLaneExit = 1 << 30;
 
 // The reference flag and the qsl_line_status of a finished direction
 // (packed into Lane::flag so that the status costs no register in the loop).
@@ -524,7 +549,6 @@ __device__ __forceinline__ void len_add(Lane<EXACT>& L, double x_exact, float x_
 template <bool EXACT, class F>
 __device__ __forceinline__ void lane_begin(const F& f, const TraceJob<F>& J, Lane<EXACT>& L, long long line, int dir,
                                            float s_len, float tol_coef, const float3 nrm, unsigned& ns) {
-    L.line = line;
     L.dsign = dir > 0 ? 0u : 0x80000000u;
     L.p = v3(__ldg(J.inp_x + line), __ldg(J.inp_y + line), __ldg(J.inp_z + line));
     L.pc = v3(0.f, 0.f, 0.f);
@@ -635,56 +659,26 @@ __device__ __forceinline__ int lane_control(const TraceJob<F>& J, Lane<EXACT>& L
     return 0;
 }
 
-template <bool EXACT, bool TWIST, class F>
-__device__ __forceinline__ bool lane_move(const F& f, const TraceJob<F>& J, Lane<EXACT>& L, float3 inc,
-                                          float3 b_at_p, bool tw_on, unsigned& ns);
-
-// One trial step of the current direction.  Returns true when the direction
-// is finished (left the box, or stopped by the length / step limit) with
-// L.out, L.flag, L.len, L.tw final.  Reference: TraceBlineAdap,
-// TraceBlineAdaptive.cu:361-421 and TraceBline, TraceBline.cu:320-373.
-template <bool EXACT, bool TWIST, class F>
-__device__ __forceinline__ bool lane_step(const F& f, const TraceJob<F>& J, Lane<EXACT>& L,
-                                          typename Lane<EXACT>::len_t len_lim, bool tw_on,
-                                          unsigned& ns) {
-    if (lane_limits(J, L, len_lim)) return true;
-    const float hd = lane_hd(L);
-    float3 inc;
-    // fast twist kernels: B at L.p comes out of the step's first sample
-    float3 b_at_p = v3(0.f, 0.f, 0.f);
-    float3* const want_b = (!EXACT && TWIST && tw_on) ? &b_at_p : nullptr;
-    if (J.prm.integrator == QSL_RKF45) {
-        float err;
-        inc = step_rkf45<EXACT>(f, L.p, hd, err, ns, want_b);
-        const int c = lane_control(J, L, err);
-        if (c != 0) return c == 2;
-    } else {
-        inc = step_rk4<EXACT>(f, L.p, hd, ns, want_b);
-    }
-    return lane_move<EXACT, TWIST>(f, J, L, inc, b_at_p, tw_on, ns);
-}
-
 // The accepted step's move: the position update (Kahan-compensated in fast
-// arithmetic), the length, the twist increment and the exit test with the
-// footpoint on the face.  True when the direction is finished.
+// arithmetic), the length, the twist increment and the inside test.  True
+// when the point left the box: L.p then stays the last point inside and
+// L.out is the one outside (lane_foot finds the footpoint).
 template <bool EXACT, bool TWIST, class F>
 __device__ __forceinline__ bool lane_move(const F& f, const TraceJob<F>& J, Lane<EXACT>& L, float3 inc,
                                           float3 b_at_p, bool tw_on, unsigned& ns) {
-    const qsl_trace_params& pr = J.prm;
     // the twist integrand at the step's start point, before the position
     // update (fewer values live during the current density's sample)
     float td = 0.f;
-    float3 b1 = v3(0.f, 0.f, 0.f), j1 = v3(0.f, 0.f, 0.f);
     if (TWIST && tw_on) {
-        j1 = J.cur_packed ? sample<EXACT>(J.cur_store, L.p, false) : sample<EXACT>(current_view(f, J.cur), L.p, false);
+        const float3 j1 =
+            J.cur_packed ? sample<EXACT>(J.cur_store, L.p, false) : sample<EXACT>(current_view(f, J.cur), L.p, false);
         if (EXACT) {
-            b1 = sample<EXACT>(f, L.p, false);
+            td = twist_density<EXACT>(j1, sample<EXACT>(f, L.p, false));
             ns += 2;
         } else {
-            b1 = b_at_p;
+            td = twist_density<EXACT>(j1, b_at_p);
             ns += 1;
         }
-        td = twist_density<EXACT>(j1, b1);
     }
     float3 p2;
     float dl;
@@ -709,114 +703,262 @@ __device__ __forceinline__ bool lane_move(const F& f, const TraceJob<F>& J, Lane
         dl = norm_fast(v3(txy.x, txy.y, tz));
     }
     len_add(L, (double)dl, dl);
-    if (TWIST && tw_on)
-        L.tw = L.tw + (EXACT ? (double)td / 4.0 / kRefPi * (double)dl : (double)(td * dl * kInv4PiF));
-    // inside test first: the full face classification only runs on exit
-    const int flag = box_inside(f, p2) ? 0 : box_exit(f, p2);
-    if (flag > 0) {
+    double dtw = 0.0;
+    if (TWIST && tw_on) {
+        dtw = EXACT ? (double)td / 4.0 / kRefPi * (double)dl : (double)(td * dl * kInv4PiF);
+        L.tw = L.tw + dtw;
+    }
+    L.steps++;
+    if (!box_inside(f, p2)) {
         len_add(L, -(double)dl, -dl);
-        if (TWIST && tw_on)
-            L.tw = L.tw - (EXACT ? (double)td / 4.0 / kRefPi * (double)dl : (double)(td * dl * kInv4PiF));
-        if (flag <= 6) {
-            const int d = (flag - 1) / 2;
-            const float q1 = comp(L.p, d), q2 = comp(p2, d);
-            float qmid = q1;
-            if ((double)fabsf(q1 - q2) > 1e-3) {
-                qmid = (flag % 2 == 1) ? 0.f : (float)f.d.n(d);
-                const float3 u1 = sample<EXACT>(f, L.p, true);
-                const float3 u2 = sample<EXACT>(f, p2, true);
-                ns += 2;
-                if (((double)fabsf(comp(u1, d)) < 0.2) | ((double)fabsf(comp(u2, d)) < 0.2)) {
-                    L.out.x = (L.p.x * (q2 - qmid) + p2.x * (qmid - q1)) / (q2 - q1);
-                    L.out.y = (L.p.y * (q2 - qmid) + p2.y * (qmid - q1)) / (q2 - q1);
-                    L.out.z = (L.p.z * (q2 - qmid) + p2.z * (qmid - q1)) / (q2 - q1);
-                } else {
-                    if constexpr (RolledStages<F>::value) L.out = step_rk4_normal_rolled<EXACT>(f, L.p, qmid - q1, d);
-                    else L.out = step_rk4_normal<EXACT>(f, L.p, qmid - q1, d);
-                    ns += 4;
-                }
-                len_add(L, (double)fabsf(qmid - q1) / (1e-4 + (double)fabsf(comp(u1, d))),
-                        fabsf(qmid - q1) / (1e-4f + fabsf(comp(u1, d))));
-                b1 = u1;
-            } else {
-                L.out = L.p;
-            }
-            if (TWIST && tw_on && pr.boundary_twist) {
-                L.tw = L.tw + (double)twist_density<EXACT>(j1, b1) / 4.0 / kRefPi * (double)fabsf(qmid - q1) /
-                                  (1e-4 + (double)fabsf(comp(b1, d)));
-            }
-        } else {
-            L.out = p2;
-        }
-        const bool finite = isfinite(p2.x) & isfinite(p2.y) & isfinite(p2.z);
-        L.flag = pack_flag(flag, flag <= 6 ? QSL_LINE_FACE : (finite ? QSL_LINE_EDGE : QSL_LINE_NAN));
-        L.p = p2;
-        L.steps++;
+        if (TWIST && tw_on) L.tw = L.tw - dtw;
+        L.out = p2;
+        L.flag = kLaneExit;
         return true;
     }
     L.p = p2;
-    L.steps++;
     return false;
 }
 
-// A finished direction's outputs, as the reference writes them
-// (TraceBlineAdaptive.cu:466-501): after the forward direction its end
-// footpoint, flag, B and length, then the backward direction begins (returns
-// true); after the backward one the start footpoint, B at the seed and
-// B_flag (returns false: the line is done).  The per-line scalars come from
-// functors so that they are re-read rather than held in registers.
-template <bool EXACT, bool TWIST, class F, class SL, class TC, class NR>
-__device__ __forceinline__ bool lane_finish(const F& f, const TraceJob<F>& J, Lane<EXACT>& L, bool tw_on,
-                                            unsigned& ns, const SL& s_len_of, const TC& tol_coef_of,
-                                            const NR& nrm_of) {
-    const long long i = L.line;
-    const TraceOut& o = J.o;
-    if (L.dsign == 0) {
-        const float3 pe = L.out;
-        const float3 be = sample_endpoint<EXACT>(f, pe);
-        ns += 1;
-        o.end_x[i] = pe.x; o.end_y[i] = pe.y; o.end_z[i] = pe.z;
-        o.flag_end[i] = lane_flag(L.flag);
-        if (o.status_end) o.status_end[i] = lane_status(L.flag);
-        o.bend_x[i] = be.x; o.bend_y[i] = be.y; o.bend_z[i] = be.z;
-        o.line_len[i] = (double)L.len;
-        if (TWIST && tw_on) o.twist[i] = L.tw;
-        lane_begin<EXACT>(f, J, L, i, -1, s_len_of(), tol_coef_of(), nrm_of(), ns);
-        return true;
+// One trial step of the current direction.  Returns true when the direction
+// is finished (left the box, or stopped by the length / step / reject limit).
+// Reference: TraceBlineAdap, TraceBlineAdaptive.cu:361-421 and TraceBline,
+// TraceBline.cu:320-373.
+template <bool EXACT, bool TWIST, class F>
+__device__ __forceinline__ bool lane_step(const F& f, const TraceJob<F>& J, Lane<EXACT>& L,
+                                          typename Lane<EXACT>::len_t len_lim, bool tw_on,
+                                          unsigned& ns) {
+    if (lane_limits(J, L, len_lim)) return true;
+    const float hd = lane_hd(L);
+    float3 inc;
+    // fast twist kernels: B at L.p comes out of the step's first sample
+    float3 b_at_p = v3(0.f, 0.f, 0.f);
+    float3* const want_b = (!EXACT && TWIST && tw_on) ? &b_at_p : nullptr;
+    if (J.prm.integrator == QSL_RKF45) {
+        float err;
+        inc = step_rkf45<EXACT>(f, L.p, hd, err, ns, want_b);
+        const int c = lane_control(J, L, err);
+        if (c != 0) return c == 2;
+    } else {
+        inc = step_rk4<EXACT>(f, L.p, hd, ns, want_b);
     }
-    const float3 ps = L.out;
-    const float3 bs = sample_endpoint<EXACT>(f, ps);
-    const float3 p0 = v3(__ldg(J.inp_x + i), __ldg(J.inp_y + i), __ldg(J.inp_z + i));
-    const float3 b0 = sample_endpoint<EXACT>(f, p0);
-    ns += 2;
-    o.start_x[i] = ps.x; o.start_y[i] = ps.y; o.start_z[i] = ps.z;
-    o.flag_start[i] = lane_flag(L.flag);
-    if (o.status_start) o.status_start[i] = lane_status(L.flag);
-    o.bstart_x[i] = bs.x; o.bstart_y[i] = bs.y; o.bstart_z[i] = bs.z;
-    o.bthis_x[i] = b0.x; o.bthis_y[i] = b0.y; o.bthis_z[i] = b0.z;
-    o.line_len[i] = o.line_len[i] + (double)L.len;
-    if (TWIST && tw_on) o.twist[i] = o.twist[i] + L.tw;
-    // B nearly in the seed plane (TraceBlineAdaptive.cu:498-501)
-    const float3 nrm = nrm_of();
-    const float bn = b0.x * nrm.x + b0.y * nrm.y + b0.z * nrm.z;
-    const float bm = sqrtf(b0.x * b0.x + b0.y * b0.y + b0.z * b0.z);
-    o.b_flag[i] = ((double)fabsf(bn) * 100. < (double)bm) ? 1 : 0;
-    return false;
+    return lane_move<EXACT, TWIST>(f, J, L, inc, b_at_p, tw_on, ns);
 }
 
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
+// The footpoint of a finished direction: the exit face of a point that left
+// the box and the line's crossing of it, with the length and twist of the
+// exit segment (TraceBlineAdaptive.cu:380-418).  Sets L.out and L.flag
+// (reference flag and qsl_line_status).  A limit's end has both already.
+template <bool EXACT, bool TWIST, class F>
+__device__ __forceinline__ void lane_foot(const F& f, const TraceJob<F>& J, Lane<EXACT>& L, bool tw_on,
+                                          unsigned& ns) {
+    if (L.flag != kLaneExit) return;
+    const float3 p2 = L.out;
+    const int flag = box_exit(f, p2);
+    if (flag <= 6) {
+        const int d = (flag - 1) / 2;
+        const float q1 = comp(L.p, d), q2 = comp(p2, d);
+        float qmid = q1;
+        float3 b1 = v3(0.f, 0.f, 0.f);
+        const bool far = (double)fabsf(q1 - q2) > 1e-3;
+        if (far) {
+            qmid = (flag % 2 == 1) ? 0.f : (float)f.d.n(d);
+            const float3 u1 = sample_outlined<EXACT>(f, L.p, true);
+            const float3 u2 = sample_outlined<EXACT>(f, p2, true);
+            ns += 2;
+            if (((double)fabsf(comp(u1, d)) < 0.2) | ((double)fabsf(comp(u2, d)) < 0.2)) {
+                L.out.x = (L.p.x * (q2 - qmid) + p2.x * (qmid - q1)) / (q2 - q1);
+                L.out.y = (L.p.y * (q2 - qmid) + p2.y * (qmid - q1)) / (q2 - q1);
+                L.out.z = (L.p.z * (q2 - qmid) + p2.z * (qmid - q1)) / (q2 - q1);
+            } else {
+                L.out = step_rk4_normal<EXACT>(f, L.p, qmid - q1, d);
+                ns += 4;
+            }
+            len_add(L, (double)fabsf(qmid - q1) / (1e-4 + (double)fabsf(comp(u1, d))),
+                    fabsf(qmid - q1) / (1e-4f + fabsf(comp(u1, d))));
+            b1 = u1;
+        } else {
+            L.out = L.p;
+        }
+        if (TWIST && tw_on && J.prm.boundary_twist) {
+            // J and (on the face already) B at the exit step's start point
+            const float3 j1 = J.cur_packed ? sample_outlined<EXACT>(J.cur_store, L.p, false)
+                                           : sample_outlined<EXACT>(current_view(f, J.cur), L.p, false);
+            if (!far) b1 = sample_outlined<EXACT>(f, L.p, false);
+            L.tw = L.tw + (double)twist_density<EXACT>(j1, b1) / 4.0 / kRefPi * (double)fabsf(qmid - q1) /
+                              (1e-4 + (double)fabsf(comp(b1, d)));
+        }
+    }
+    const bool finite = isfinite(p2.x) & isfinite(p2.y) & isfinite(p2.z);
+    L.flag = pack_flag(flag, flag <= 6 ? QSL_LINE_FACE : (finite ? QSL_LINE_EDGE : QSL_LINE_NAN));
 }
 
-// The tracer kernel.  QUEUE = true: persistent grid; each warp takes chunks
-// of J.chunk consecutive lines from the device counter J.queue and its lanes
-// refill from the warp's current chunk the moment their line ends, so a
-// warp's lanes stay on neighbouring seeds (spatially coherent gathers) while
-// uneven line lengths never idle them.  QUEUE = false: line = global thread
-// index + k * total threads.  Lines are visited in J.order when it is set.
-// TWIST compiles the twist integral in; it runs when the runtime flag is set.
+// The second direction of a line: from the seed again with the first step
+// size and the same tolerance (it depends on the seed alone).
+template <bool EXACT, class F>
+__device__ __forceinline__ void lane_turn(const TraceJob<F>& J, Lane<EXACT>& L, long long line, float s_len,
+                                          unsigned& ns) {
+    L.dsign = 0x80000000u;
+    L.p = v3(__ldg(J.inp_x + line), __ldg(J.inp_y + line), __ldg(J.inp_z + line));
+    L.pc = v3(0.f, 0.f, 0.f);
+    L.h = s_len;
+    L.len = 0;
+    L.lc = 0.f;
+    L.tw = 0.0;
+    L.steps = 0;
+    L.rej = 0;
+    if (J.prm.integrator == QSL_RKF45) ns += 1;  // the tolerance's sample counts for both directions
+}
+
+// What a finished direction leaves behind until its warp's other lanes are
+// done (lane_foot and the outputs then run once for the whole warp): an
+// array per lane, one row per direction.  Indexed by the direction it lives
+// in local memory, which the stepping loop does not touch (as 4.6 KB of
+// shared memory per block it took 4 % off the L1-bound Q cube, 113.4 ->
+// 117.7 ms).
+template <bool EXACT>
+struct Stash {
+    float p[3], q[3];
+    int code;
+    float lc;
+    typename Lane<EXACT>::len_t len;
+    double tw;
+};
+template <bool EXACT, bool TWIST>
+__device__ __forceinline__ void stash_put(Stash<EXACT>& S, const Lane<EXACT>& L) {
+    S.p[0] = L.p.x; S.p[1] = L.p.y; S.p[2] = L.p.z;
+    S.q[0] = L.out.x; S.q[1] = L.out.y; S.q[2] = L.out.z;
+    S.code = L.flag;
+    S.lc = L.lc;
+    S.len = L.len;
+    if (TWIST) S.tw = L.tw;
+}
+template <bool EXACT, bool TWIST>
+__device__ __forceinline__ void stash_get(const Stash<EXACT>& S, Lane<EXACT>& L) {
+    L.p = v3(S.p[0], S.p[1], S.p[2]);
+    L.out = v3(S.q[0], S.q[1], S.q[2]);
+    L.flag = S.code;
+    L.lc = S.lc;
+    L.len = S.len;
+    if (TWIST) L.tw = S.tw;
+}
+// the two warps of a split pair wait for each other (64 threads, a barrier
+// of their own).  The barrier's number is a constant on each side: a number
+// from a register reserves all sixteen for the block, and the SM then holds
+// four blocks.
+__device__ __forceinline__ void pair_sync() {
+    static_assert(kTraceThreads == 128, "two pairs of warps per block");
+    __syncwarp();
+    __threadfence_block();
+    if (threadIdx.x < 64) asm volatile("bar.sync 1, 64;" ::: "memory");
+    else asm volatile("bar.sync 2, 64;" ::: "memory");
+}
+
+// The end of a warp's lines, for all its lanes at once: the footpoints and
+// samples of B of the directions in S and the outputs.
+template <bool EXACT, bool TWIST, class F>
+__device__ __forceinline__ unsigned lines_finish(const F& f, const TraceJob<F>& J, const Stash<EXACT>* S, long long i,
+                                         bool valid, bool split, float3 nrm, bool tw_on) {
+    Lane<EXACT> L;
+    unsigned ns = 0;
+    const TraceOut& o = J.o;
+    const bool back_only = split && ((threadIdx.x >> 5) & 1);
+    double len = 0.0, tw = 0.0;
+    if (valid) {
+        const float3 p0 = v3(__ldg(J.inp_x + i), __ldg(J.inp_y + i), __ldg(J.inp_z + i));
+#pragma unroll 1
+        for (int dir = back_only ? 1 : 0; dir < (split && !back_only ? 1 : 2); ++dir) {
+            stash_get<EXACT, TWIST>(S[dir], L);
+            const bool fwd = dir == 0;
+            lane_foot<EXACT, TWIST>(f, J, L, tw_on, ns);
+            const float3 foot = L.out;
+            const float3 b = sample_endpoint<EXACT>(f, foot);
+            ns += 1;
+            // the end footpoint's arrays forward, the start's backward
+            (fwd ? o.end_x : o.start_x)[i] = foot.x;
+            (fwd ? o.end_y : o.start_y)[i] = foot.y;
+            (fwd ? o.end_z : o.start_z)[i] = foot.z;
+            (fwd ? o.flag_end : o.flag_start)[i] = lane_flag(L.flag);
+            int* const st = fwd ? o.status_end : o.status_start;
+            if (st) st[i] = lane_status(L.flag);
+            (fwd ? o.bend_x : o.bstart_x)[i] = b.x;
+            (fwd ? o.bend_y : o.bstart_y)[i] = b.y;
+            (fwd ? o.bend_z : o.bstart_z)[i] = b.z;
+            len = (fwd | back_only) ? (double)L.len : len + (double)L.len;
+            if (TWIST && tw_on) tw = (fwd | back_only) ? L.tw : tw + L.tw;
+        }
+        if (!split | back_only) {
+            const float3 b0 = sample_endpoint<EXACT>(f, p0);
+            ns += 1;
+            o.bthis_x[i] = b0.x; o.bthis_y[i] = b0.y; o.bthis_z[i] = b0.z;
+            // B nearly in the seed plane (TraceBlineAdaptive.cu:498-501)
+            const float bn = b0.x * nrm.x + b0.y * nrm.y + b0.z * nrm.z;
+            const float bm = sqrtf(b0.x * b0.x + b0.y * b0.y + b0.z * b0.z);
+            o.b_flag[i] = ((double)fabsf(bn) * 100. < (double)bm) ? 1 : 0;
+        }
+    }
+    if (split) {
+        // the backward warp's length and twist through the output arrays
+        if (valid & back_only) {
+            o.line_len[i] = len;
+            if (TWIST && tw_on) o.twist[i] = tw;
+        }
+        pair_sync();
+        if (valid & !back_only) {
+            len = len + __ldcg(o.line_len + i);
+            if (TWIST && tw_on) tw = tw + __ldcg(o.twist + i);
+        }
+    }
+    if (valid & !back_only) {
+        o.line_len[i] = len;
+        if (TWIST && tw_on) o.twist[i] = tw;
+    }
+    return ns;
+}
+
+// One line per lane of a warp, the lanes in lockstep: seed `i` of every lane
+// that has one (`valid`), forward, then backward.  A lane whose direction
+// ends goes on with its next one at once but leaves the footpoint, the
+// samples of B and the outputs to the end, where the whole warp does them
+// together: done as each lane ends, they ran for one or two lanes at a time
+// (7-9 samples per direction, 32 times over).
+//
+// split: warps 2k and 2k + 1 of a block hold the same 32 lines, the first
+// forward and the second backward, and the pair adds the two lengths (and
+// twists) up at the end.  A line's directions depend on each other in
+// nothing else, and a launch that leaves the GPU's warp slots half empty
+// lasts as long as its longest line.
+//
+// The per-line scalars come from functors so that they are re-read where
+// they are used rather than held in registers through the stepping loop.
+template <bool EXACT, bool TWIST, class F, class SL, class TC, class NR>
+__device__ __forceinline__ void trace_lines(const F& f, const TraceJob<F>& J, long long i, bool valid,
+                                            bool split, typename Lane<EXACT>::len_t len_lim, const SL& s_len_of,
+                                            const TC& tol_coef_of, const NR& nrm_of, bool tw_on, unsigned& ns) {
+    Lane<EXACT> L;
+    Stash<EXACT> S[2];
+    if (valid) {
+        lane_begin<EXACT>(f, J, L, i, split && ((threadIdx.x >> 5) & 1) ? -1 : 1, s_len_of(), tol_coef_of(), nrm_of(),
+                          ns);
+        while (true) {
+            if (!lane_step<EXACT, TWIST>(f, J, L, len_lim, tw_on, ns)) continue;
+            stash_put<EXACT, TWIST>(S[L.dsign >> 31], L);
+            if (split | (L.dsign != 0)) break;
+            lane_turn(J, L, i, s_len_of(), ns);
+        }
+    }
+    __syncwarp();
+    ns += lines_finish<EXACT, TWIST>(f, J, S, i, valid, split, nrm_of(), tw_on);
+}
+
+// The tracer kernel: every warp takes 32 lines at a time and traces them in
+// lockstep.  QUEUE = true: persistent grid; a warp takes chunks of J.chunk
+// consecutive lines from the device counter J.queue, so uneven lines even
+// out over the warps.  QUEUE = false: line = global thread index + k * total
+// threads.  A launch whose grid has two threads per line splits the
+// directions over warp pairs (trace_lines).  Lines are visited in J.order
+// when it is set.  TWIST compiles the twist integral in; it runs when the
+// runtime flag is set.
 template <bool EXACT, bool TWIST, bool QUEUE, class F>
 __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
     F f = J.f;
@@ -842,8 +984,10 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
         return J.s.cross_dev ? v3(__ldg(J.s.cross_dev), __ldg(J.s.cross_dev + 1), __ldg(J.s.cross_dev + 2))
                              : v3(J.s.cross[0], J.s.cross[1], J.s.cross[2]);
     };
-    long long n = J.s.n_dev ? (long long)__ldg(J.s.n_dev) : J.s.n;
-    if (J.s.n_cap >= 0 && n > J.s.n_cap) n = J.s.n_cap;
+    auto n_of = [&J]() {
+        const long long n = J.s.n_dev ? (long long)__ldg(J.s.n_dev) : J.s.n;
+        return J.s.n_cap >= 0 && n > J.s.n_cap ? (long long)J.s.n_cap : n;
+    };
     const bool tw_on = TWIST && (J.s.twist_flag_dev ? *J.s.twist_flag_dev : (J.s.twist_on != 0));
     if (!store_active(f)) return;
     store_prepare(f);
@@ -860,83 +1004,40 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
         len_lim = (typename Lane<EXACT>::len_t)(J.prm.len_ratio * len_scale(f));
     unsigned ns = 0;
     const int lane_id = threadIdx.x & 31;
-
-    Lane<EXACT> L;
-    bool active = false;
-    bool drained = false;
-    // warp-uniform chunk window [c_next, c_end) of the work queue
-    long long c_next = 0, c_end = 0;
-    bool q_empty = false;
-    // lines per refill: the caller's choice, else an even share per warp of
-    // the grid between one warp's width (a small launch then uses every warp:
-    // with 256 the 128 x 128 plane ran on 64 of 2432 warps) and 256 (the
-    // neighbouring seeds that keep a warp's gathers together)
-    long long chunk = J.chunk;
-    if (QUEUE && chunk <= 0) {
-        const long long warps = (long long)gridDim.x * (blockDim.x / 32);
-        chunk = ((n + warps - 1) / warps + 31) / 32 * 32;
-        chunk = chunk < 32 ? 32 : (chunk > 256 ? 256 : chunk);
-    }
-    long long next_static = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-
+    const bool split = 2 * n_of() <= (long long)gridDim.x * blockDim.x;
+    const bool queued = QUEUE && !split;
+    // the warp's first line, and the end of its chunk
+    long long line = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane_id, end = 0;
+    if (split) line = (line >> 6) * 32;
+    if (queued) line = 0;
     while (true) {
-        // ---- give lanes without a line the next ones ----
-        if (QUEUE) {
-            bool need = !active && !drained;
-            unsigned m = __ballot_sync(0xffffffffu, need);
-            while (m) {
-                if (c_next >= c_end) {
-                    if (q_empty) {
-                        drained = drained || need;
-                        break;
-                    }
-                    unsigned long long base = 0;
-                    if (lane_id == 0) base = atomicAdd(J.queue, (unsigned long long)chunk);
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    if ((long long)base >= n) {
-                        q_empty = true;
-                        drained = drained || need;
-                        break;
-                    }
-                    c_next = (long long)base;
-                    c_end = min((long long)base + chunk, n);
-                }
-                const long long avail = c_end - c_next;
-                const int take = (int)min((long long)__popc(m), avail);
-                const int rank = __popc(m & lanemask_lt());
-                if (need && rank < take) {
-                    const long long line = c_next + rank;
-                    const long long sidx = J.order ? (long long)__ldg(J.order + line) : line;
-                    lane_begin<EXACT>(f, J, L, sidx, +1, s_len_of(), tol_coef_of(), nrm_of(), ns);
-                    active = true;
-                    need = false;
-                }
-                c_next += take;
-                m = __ballot_sync(0xffffffffu, need);
+        if (queued && line >= end) {
+            // lines per turn of the queue: the caller's choice, else an even
+            // share per warp of the grid between one warp's width (a small
+            // launch then uses every warp: with 256 the 128 x 128 plane ran
+            // on 64 of 2432 warps) and 256
+            long long chunk = J.chunk;
+            if (chunk <= 0) {
+                const long long warps = (long long)gridDim.x * (kTraceThreads / 32);
+                chunk = ((n_of() + warps - 1) / warps + 31) / 32 * 32;
+                chunk = chunk < 32 ? 32 : (chunk > 256 ? 256 : chunk);
             }
-            if (!__any_sync(0xffffffffu, active)) break;
-            if (!active) continue;
-        } else {
-            if (!active) {
-                if (next_static >= n) break;
-                const long long sidx = J.order ? (long long)__ldg(J.order + next_static) : next_static;
-                lane_begin<EXACT>(f, J, L, sidx, +1, s_len_of(), tol_coef_of(), nrm_of(), ns);
-                next_static += (long long)gridDim.x * blockDim.x;
-                active = true;
-            }
+            unsigned long long base = 0;
+            if (lane_id == 0) base = atomicAdd(J.queue, (unsigned long long)chunk);
+            line = (long long)__shfl_sync(0xffffffffu, base, 0);
+            end = min(line + chunk, n_of());
         }
-
-        // ---- advance this lane's line by one trial step ----
-        if (lane_step<EXACT, TWIST>(f, J, L, len_lim, tw_on, ns)) {
-            // a lane's sample count nears 32 bits: hand it over (checked at
-            // direction ends only; exact while one direction takes fewer than
-            // 5e8 trial steps)
-            if (ns > (1u << 30)) {
-                if (J.samples) atomicAdd(J.samples, (unsigned long long)ns);
-                ns = 0;
-            }
-            active = lane_finish<EXACT, TWIST>(f, J, L, tw_on, ns, s_len_of, tol_coef_of, nrm_of);
+        if (line >= n_of()) break;
+        const bool valid = line + lane_id < (queued ? end : n_of());
+        const long long i = (valid && J.order) ? (long long)__ldg(J.order + line + lane_id) : line + lane_id;
+        trace_lines<EXACT, TWIST>(f, J, i, valid, split, len_lim, s_len_of, tol_coef_of, nrm_of, tw_on, ns);
+        // a lane's sample count nears 32 bits: hand it over (exact while one
+        // line takes fewer than 5e8 trial steps)
+        if (ns > (1u << 30)) {
+            if (J.samples) atomicAdd(J.samples, (unsigned long long)ns);
+            ns = 0;
         }
+        line += queued ? 32 : (long long)gridDim.x * blockDim.x / (split ? 2 : 1);
     }
     if (J.samples) {
         // one atomic per warp (blocks are whole warps; every lane gets here)

@@ -11,7 +11,7 @@
 namespace qsl {
 
 template <bool TWIST, bool QUEUE, class F>
-__global__ void __launch_bounds__(kTraceBlock) k_trace_exact(const TraceJob<F> J) {
+__global__ void __launch_bounds__(kTraceBlock) k_trace_exact(const __grid_constant__ TraceJob<F> J) {
     trace_kernel_body<true, TWIST, QUEUE>(J);
 }
 
@@ -20,13 +20,8 @@ static cudaError_t launch_exact(const TraceJob<F>& J, bool twist, Schedule sched
     const bool q = sched == SCHED_QUEUE;
     const void* k = q ? (twist ? (const void*)k_trace_exact<true, true, F> : (const void*)k_trace_exact<false, true, F>)
                       : (twist ? (const void*)k_trace_exact<true, false, F> : (const void*)k_trace_exact<false, false, F>);
-    int grid;
-    if (q) {
-        grid = persistent_grid(k, kTraceBlock);
-    } else {
-        long long g = (n_host + kTraceBlock - 1) / kTraceBlock;
-        grid = (int)(g < 1 ? 1 : (g > (1 << 30) ? (1 << 30) : g));
-    }
+    int grid = persistent_grid(k, kTraceBlock);
+    if (!q) grid = static_grid(n_host, grid);
     if (grid <= 0) return cudaErrorInvalidConfiguration;
     if (q) {
         if (twist) k_trace_exact<true, true, F><<<grid, kTraceBlock, 0, st>>>(J);

@@ -188,7 +188,7 @@ int qsl_field_update(qsl_field_t *field, const float *Bx, const float *By, const
  * (TraceBlineAdaptive.cu:429-510).
  * ------------------------------------------------------------------------ */
 enum qsl_schedule {
-    QSL_SCHED_QUEUE = 0, /* persistent grid, per-lane refill from a device work counter */
+    QSL_SCHED_QUEUE = 0, /* persistent grid, warps take lines from a device work counter */
     QSL_SCHED_STATIC = 1 /* one line per thread; the grid covers n (with n_dev set, n is the capacity) */
 };
 
@@ -211,7 +211,7 @@ typedef struct qsl_trace_io {
 /* Scheduling of a trace launch (host struct; pointers are device pointers). */
 typedef struct qsl_sched {
     int32_t schedule;            /* qsl_schedule */
-    int32_t chunk;               /* QUEUE: lines a warp takes per refill (0 = 256) */
+    int32_t chunk;               /* QUEUE: lines a warp takes at a time (0 = chosen from n) */
     const uint32_t *order;       /* optional: line k traces seed order[k] and writes its outputs at
                                     order[k] (a permutation of [0, n)); visiting seeds in compact
                                     tiles keeps a warp's gathers coherent */
