@@ -424,11 +424,12 @@ class QMapPlan:
     (float64).  Reference workflow: demo/Q_RKF45CuPy3D.ipynb cell 7 and
     demo/Q_RKF45CuPy.ipynb cells 7-11."""
 
-    # measured best per field layout on GB300 (trace of the 512x512x256 cube):
-    # register budget for 7 resident blocks/SM for the brick store (FP32
-    # interpolation), 8 for the cell-record and float4 stores, the compiler's
-    # choice for SoA
-    DEFAULT_OCCUPANCY = {"h8c": 8, "h4b": 7, "f4": 8, "soa": 0}
+    # resident blocks per SM of each layout's kernels, measured on GB300 (ms on
+    # 131 x 147 x 12 / 258 x 514 x 1 seeds): bricks 1.50 / 0.87 at 6 against
+    # 1.61 / 1.01 at 7; cell records 1.63 / 1.17 at 7 (1.69 / 1.13 at 6);
+    # float4 and SoA with the compiler's own registers (0: 3-4 blocks, no
+    # spills), 2.13 / 0.93 against 2.67 / 1.13 at 8 for float4
+    DEFAULT_OCCUPANCY = {"h8c": 7, "h4b": 6, "f4": 0, "soa": 0}
 
     def __init__(self, n0, n1, nplanes=1, device="cuda", pseudo=True, tile=(8, 8), chunk=256, schedule="static",
                  occupancy=None, hybrid=False):
@@ -653,7 +654,7 @@ class PlaneQBatch:
             n0, n1, npl = int(j["n0"]), int(j["n1"]), int(j.get("nplanes", 1))
             qn = npl * (n0 - 2) * (n1 - 2)
             self.Q.append(self.workspace[off:off + 8 * qn].view(torch.float64).view(npl, n0 - 2, n1 - 2))
-        # register budget of the batched kernels (resident blocks per SM; 0 = 8)
+        # register budget of the batched kernels (resident blocks per SM; 0 = 6)
         self.occupancy = 0
 
     @property
@@ -824,7 +825,7 @@ class BatchPlan:
         """Lines [lo, hi) of the batch (hi < 0: all); max_blocks > 0: at most
         that many resident blocks (they loop over the lines), leaving the rest
         of the GPU's block slots free; occupancy: the kernels' register budget
-        in resident blocks per SM (6-10, 0 = 8)."""
+        in resident blocks per SM (6-10, 0 = 6)."""
         _lib.check(_lib.load().qsl_batch_run_window(self._dev.data_ptr(), ctypes.byref(self.info), ptr(samples),
                                                     int(lo), int(hi), int(max_blocks), int(occupancy),
                                                     stream_handle(stream)),
@@ -908,7 +909,7 @@ class QBatch:
         self.sub_batch = BatchPlan(sub_jobs, stream=stream)
         self.graph = None
         # register budget of the batched kernels (resident blocks per SM;
-        # autotune.tune_batch measures the choices; 0 = 8)
+        # autotune.tune_batch measures the choices; 0 = 6)
         self.occupancy = 0
 
     @property

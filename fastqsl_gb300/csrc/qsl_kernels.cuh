@@ -99,11 +99,11 @@ static const void* batch_kernel_minb(bool twist) {
 template <class F>
 static const void* batch_kernel(int occupancy, bool twist) {
     switch (occupancy) {
-        case 6: return batch_kernel_minb<F, 6>(twist);
         case 7: return batch_kernel_minb<F, 7>(twist);
+        case 8: return batch_kernel_minb<F, 8>(twist);
         case 9: return batch_kernel_minb<F, 9>(twist);
         case 10: return batch_kernel_minb<F, 10>(twist);
-        default: return batch_kernel_minb<F, 8>(twist);
+        default: return batch_kernel_minb<F, 6>(twist);
     }
 }
 
@@ -120,11 +120,11 @@ static cudaError_t launch_batch(const TraceJob<F>* jobs, const long long* begin,
     int grid = static_grid(line_hi - line_lo, resident);
     if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;  // the grid-stride loop covers the rest
     switch (occupancy) {
-        case 6: launch_batch_minb<F, 6>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
         case 7: launch_batch_minb<F, 7>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
         case 9: launch_batch_minb<F, 9>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
         case 10: launch_batch_minb<F, 10>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
-        default: launch_batch_minb<F, 8>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
+        case 8: launch_batch_minb<F, 8>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
+        default: launch_batch_minb<F, 6>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
     }
     return cudaGetLastError();
 }

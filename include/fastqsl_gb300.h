@@ -286,7 +286,7 @@ int qsl_batch_pack(const qsl_batch_job *jobs_h, int njobs, void *table_h, int64_
  * never share the GPU with more than a window of it, and caps its resident
  * blocks below the GPU's capacity.  occupancy: the register budget of the
  * batched kernels, for this many resident 128-thread blocks per SM (6-10;
- * 0 = 8). */
+ * 0 = 6). */
 int qsl_batch_run_window(const void *table_dev, const qsl_batch_info *info_h, unsigned long long *samples_dev,
                          int64_t line_lo, int64_t line_hi, int max_blocks, int occupancy, qsl_stream_t stream);
 int qsl_batch_run(const void *table_dev, const qsl_batch_info *info_h, unsigned long long *samples_dev,
