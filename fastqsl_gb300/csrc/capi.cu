@@ -1199,6 +1199,22 @@ int qsl_curl_grid(const float* Bx, const float* By, const float* Bz, int nx, int
     return QSL_OK;
 }
 
+int qsl_trace_path_both(const float* Bx, const float* By, const float* Bz, int nx, int ny, int nz,
+                        const double* seeds, int64_t n, int64_t mid, double dr, float* out_x, float* out_y,
+                        float* out_z, int64_t out_len, qsl_stream_t stream) {
+    if (n < 0 || out_len < 0) return fail(QSL_ERR_INVALID, "negative count");
+    if (n == 0) return QSL_OK;
+    if (!Bx || !By || !Bz || !seeds || !out_x || !out_y || !out_z) return fail(QSL_ERR_INVALID, "null argument");
+    if (!dims_ok(nx, ny, nz)) return fail(QSL_ERR_INVALID, "bad field shape %d x %d x %d", nx, ny, nz);
+    if (n > (int64_t)1 << 36) return fail(QSL_ERR_TOO_LARGE, "too many seeds");
+    if (out_len == 0) return QSL_OK;
+    if (mid < 0 || mid >= out_len) return fail(QSL_ERR_INVALID, "seed index outside the output rows");
+    QSL_CHECK_CUDA(launch_trace_path_both(Bx, By, Bz, nx, ny, nz, seeds, n, mid, dr, out_x, out_y, out_z, out_len,
+                                          (cudaStream_t)stream),
+                   "trace path");
+    return QSL_OK;
+}
+
 int qsl_trace_path(const float* Bx, const float* By, const float* Bz, int nx, int ny, int nz, const double* seeds,
                    int64_t n, int64_t start, int64_t stop, int64_t stride, double dr, float* out_x, float* out_y,
                    float* out_z, int64_t out_len, qsl_stream_t stream) {

@@ -93,6 +93,9 @@ cudaError_t launch_curl(const float* bx, const float* by, const float* bz, const
 cudaError_t launch_trace_path(const float* bx, const float* by, const float* bz, int nx, int ny, int nz,
                               const double* seeds, long long n, long long start, long long stop, long long stride,
                               double dr, float* ox, float* oy, float* oz, long long out_len, cudaStream_t st);
+cudaError_t launch_trace_path_both(const float* bx, const float* by, const float* bz, int nx, int ny, int nz,
+                                   const double* seeds, long long n, long long mid, double dr, float* ox, float* oy,
+                                   float* oz, long long out_len, cudaStream_t st);
 cudaError_t launch_sample_points(const float* bx, const float* by, const float* bz, int nx, int ny, int nz,
                                  const double* pts, long long n, int normalize, double* out, cudaStream_t st);
 

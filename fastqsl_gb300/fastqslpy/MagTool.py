@@ -109,7 +109,7 @@ def RK4_bline(Bx, By, Bz, PP0, xl, yl, zl, steprange, dr=0.25, nk=np):
 
 
 def TraceBlines(Bx, By, Bz, seeds, maxstep=2e4, dr=0.25):
-    """TraceBline for many seeds (n, 3) in one pair of launches; returns
+    """TraceBline for many seeds (n, 3) in one launch; returns
     (xlines, ylines, zlines) float32 arrays of shape (n, maxstep), NaN where
     a line has no point.  Unlike TraceBline, the step is `dr` (forward +dr,
     backward -dr)."""
@@ -119,8 +119,11 @@ def TraceBlines(Bx, By, Bz, seeds, maxstep=2e4, dr=0.25):
     mid = int(maxstep / 2)
     s = torch.tensor(np.asarray(seeds, np.float64).reshape(-1, 3), device=dev)
     out = torch.full((3, s.shape[0], maxstep), float("nan"), dtype=torch.float32, device=dev)
-    _trace(B, s, out, mid, maxstep, 1, abs(dr))
-    _trace(B, s, out, mid, 0, -1, -abs(dr))
+    nx, ny, nz = (int(v) for v in B[0].shape)
+    _lib.check(_lib.load().qsl_trace_path_both(B[0].data_ptr(), B[1].data_ptr(), B[2].data_ptr(), nx, ny, nz,
+                                               s.data_ptr(), int(s.shape[0]), mid, abs(float(dr)),
+                                               out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr(), maxstep,
+                                               stream_handle()), "qsl_trace_path_both")
     r = out.cpu().numpy()
     return r[0], r[1], r[2]
 

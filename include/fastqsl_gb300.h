@@ -401,6 +401,13 @@ int qsl_trace_path(const float *Bx, const float *By, const float *Bz, int nx, in
                    int64_t n, int64_t start, int64_t stop, int64_t stride, double dr, float *out_x, float *out_y,
                    float *out_z, int64_t out_len, qsl_stream_t stream);
 
+/* TraceBline for n seeds at once: both directions of qsl_trace_path in one
+ * launch, indices mid, mid + 1, ..., out_len - 1 with step dr and mid,
+ * mid - 1, ..., 1 with step -dr (0 <= mid < out_len). */
+int qsl_trace_path_both(const float *Bx, const float *By, const float *Bz, int nx, int ny, int nz,
+                        const double *seeds, int64_t n, int64_t mid, double dr, float *out_x, float *out_y,
+                        float *out_z, int64_t out_len, qsl_stream_t stream);
+
 /* trilerp (normalize = 0) or Bnorm (normalize = 1) at n points (device
  * float64, n x 3) with MagTool's clamping; out: device float64, n x 3. */
 int qsl_sample_points(const float *Bx, const float *By, const float *Bz, int nx, int ny, int nz, const double *pts,
