@@ -208,9 +208,9 @@ __device__ __forceinline__ double over_sqrt(double a, double s) {
     g = __fma_rn(g, e, g);
     y = __fma_rn(y, e, y);
     const double d = __fma_rn(-g, g, s), h = nudge(y, -(1 << 20));
-    const double r = __fma_rn(d, h, g), r2 = __fma_rn(d, nudge(h, 1), g);
+    const double r = __fma_rn(d, nudge(h, 1), g), r2 = __fma_rn(d, nudge(h, -1), g);
     const double q = __dmul_rn(a, y), m = __fma_rn(-q, r, a);
-    const double u = __fma_rn(m, y, q), u2 = __fma_rn(m, nudge(y, 1), q);
+    const double u = __fma_rn(m, nudge(y, 1), q), u2 = __fma_rn(m, nudge(y, -1), q);
     // s in [2^-500, 2^500]: no step over- or underflows
     const int ex = (__double2hiint(s) >> 20) - 1023;
     const bool sure = (r == r2) & (u == u2) & (ex >= -500) & (ex <= 500);
@@ -221,7 +221,7 @@ __device__ __forceinline__ double over_sqrt(double a, double s) {
 __device__ __forceinline__ double sixth(double x) {
     const double y = 1.0 / 6.0;
     const double q = __dmul_rn(x, y), m = __fma_rn(-6.0, q, x);
-    const double u = __fma_rn(m, y, q), u2 = __fma_rn(m, nudge(y, 1), q);
+    const double u = __fma_rn(m, nudge(y, 1), q), u2 = __fma_rn(m, nudge(y, -1), q);
     const int ex = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
     return (u == u2) & (ex >= -500) & (ex <= 500) ? u : __ddiv_rn(x, 6.0);
 }

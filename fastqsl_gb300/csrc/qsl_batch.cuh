@@ -33,7 +33,7 @@ __device__ __forceinline__ void batch_line(const TraceJob<F>& J, long long line,
     else
         len_lim = (float)(J.prm.len_ratio * len_scale(f));
     trace_lines<false, TWIST>(
-        f, J, i, valid, split, len_lim, [&J]() { return J.s.s_len; }, [&J]() { return J.s.tol_coef; },
+        f, J, i, valid, split, LenLimit<false>{len_lim, 0.f}, [&J]() { return J.s.s_len; }, [&J]() { return J.s.tol_coef; },
         [&J]() { return v3(J.s.cross[0], J.s.cross[1], J.s.cross[2]); }, tw_on, ns);
 }
 

@@ -57,11 +57,17 @@ __device__ __forceinline__ float3 along(float3 u, const float3 g[3]) {
 }
 
 // Unit field and its gradient by central differences of the unit field at
-// p +- 1e-3 e_j.  Exact arithmetic: the offset applied in double and
-// narrowed, as `x -= 0.001` on a float does, and the difference divided by
+// p +- 1e-3 e_j.  Exact arithmetic: the offset rounded as in double and
+// narrowed (as `x -= 0.001` on a float does), and the difference divided by
 // 0.002f.  Fast arithmetic: the offset 0.001f added in float and the
 // difference multiplied by 500 (rounding-level differences; no FP64 add or
 // IEEE divide, nine of each per right-hand side otherwise).
+struct PlusMilli {
+    static constexpr double value = 0.001;
+};
+struct MinusMilli {
+    static constexpr double value = -0.001;
+};
 template <bool EXACT, class F>
 __device__ __forceinline__ float3 unit_and_grad_fd(const F& f, float3 p, float3 g[3], unsigned& ns) {
     const float3 b = sample<EXACT>(f, p, true);
@@ -74,9 +80,11 @@ __device__ __forceinline__ float3 unit_and_grad_fd(const F& f, float3 p, float3 
     for (int j = 0; j < 3; ++j) {
         float3 lo = p, hi = p;
         if (EXACT) {
-            if (j == 0) { lo.x = (float)((double)lo.x - 0.001); hi.x = (float)((double)hi.x + 0.001); }
-            if (j == 1) { lo.y = (float)((double)lo.y - 0.001); hi.y = (float)((double)hi.y + 0.001); }
-            if (j == 2) { lo.z = (float)((double)lo.z - 0.001); hi.z = (float)((double)hi.z + 0.001); }
+            const float c = comp(p, j);
+            const float a = add_const_exact(c, MinusMilli{}), b = add_const_exact(c, PlusMilli{});
+            if (j == 0) { lo.x = a; hi.x = b; }
+            if (j == 1) { lo.y = a; hi.y = b; }
+            if (j == 2) { lo.z = a; hi.z = b; }
         } else {
             if (j == 0) { lo.x = lo.x - 0.001f; hi.x = hi.x + 0.001f; }
             if (j == 1) { lo.y = lo.y - 0.001f; hi.y = hi.y + 0.001f; }
@@ -84,7 +92,11 @@ __device__ __forceinline__ float3 unit_and_grad_fd(const F& f, float3 p, float3 
         }
         const float3 b1 = sample<EXACT>(f, lo, true);
         const float3 b2 = sample<EXACT>(f, hi, true);
-        g[j] = EXACT ? (b2 - b1) / 0.002f : 500.f * (b2 - b1);
+        const float3 db = b2 - b1;
+        if (EXACT)
+            g[j] = v3(div_const_exact(db.x, 0.002f, 1.f / 0.002f), div_const_exact(db.y, 0.002f, 1.f / 0.002f),
+                      div_const_exact(db.z, 0.002f, 1.f / 0.002f));
+        else g[j] = 500.f * db;
     }
     ns += 7;
     return b;

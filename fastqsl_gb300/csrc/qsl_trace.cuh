@@ -94,7 +94,7 @@ struct TraceJob {
     unsigned long long* queue;    // work counter, zero at launch; null = static
     unsigned long long* samples;  // optional: total field samples
     const unsigned* order;        // optional: line k traces seed order[k] and writes its outputs there
-    int chunk;                    // lines a warp takes from the queue at a time (QUEUE; 0 = chosen from n)
+    int chunk;                    // lines a warp takes from the queue at a time (QUEUE; 0 = 32)
     int occupancy;                // resident-block variant of the fast kernels (0 = default)
 };
 
@@ -217,13 +217,20 @@ __device__ __forceinline__ float3 step_rkf45_fast_rolled(const F& f, float3 p, f
 // its term to the sums still to come, which is that order.  (Unrolled, the
 // exact samples do not fit the instruction cache: drop-in planes 18-35 %
 // slower.)
-template <class F>
-__device__ __forceinline__ float3 step_rkf45_exact(const F& f, float3 p, float h, float& err, unsigned& ns) {
+// aside(st) runs at the start of stage st: work whose results are not needed
+// in the step (Lane's pending sums), placed where the stage's sample hides
+// its latency.
+struct Nothing {
+    __device__ __forceinline__ void operator()(int) const {}
+};
+template <class F, class A>
+__device__ __forceinline__ float3 step_rkf45_exact(const F& f, float3 p, float h, float& err, unsigned& ns, A& aside) {
     const float3 zero = v3(0.f, 0.f, 0.f);
     float3 slot[5] = {zero, zero, zero, zero, zero};
     float3 sol = zero, e = zero;
 #pragma unroll 1
     for (int st = 0; st < 6; ++st) {
+        aside(st);
         const float3 k = h * sample<true>(f, st > 0 ? p + slot[0] : p, true);
 #pragma unroll
         for (int i = 0; i < 5; ++i) {
@@ -239,31 +246,43 @@ __device__ __forceinline__ float3 step_rkf45_exact(const F& f, float3 p, float h
     return sol;
 }
 
-template <bool EXACT, class F>
-__device__ __forceinline__ float3 step_rkf45(const F& f, float3 p, float h, float& err, unsigned& ns,
-                                            float3* b_raw = nullptr) {
-    if constexpr (EXACT) return step_rkf45_exact(f, p, h, err, ns);
+template <bool EXACT, class F, class A>
+__device__ __forceinline__ float3 step_rkf45(const F& f, float3 p, float h, float& err, unsigned& ns, float3* b_raw,
+                                            A& aside) {
+    if constexpr (EXACT) return step_rkf45_exact(f, p, h, err, ns, aside);
     else if constexpr (RolledStages<F>::value) return step_rkf45_fast_rolled(f, p, h, err, ns, b_raw);
     else return step_rkf45_fast(f, p, h, err, ns, b_raw);
 }
 
 // Classic RK4 on b (RK4, TraceBlineAdaptive.cu:259-267); returns the
 // increment.  The 1/6 factor is formed as (1./6.)*h in double and narrowed.
-template <bool EXACT, class F>
-__device__ __forceinline__ float3 step_rk4(const F& f, float3 p, float h, unsigned& ns, float3* b_raw = nullptr) {
+// (float)((1. / 6.) * (double)h) without the FP64 pipe: h times the double
+// 1/6 held as two floats.
+__device__ __forceinline__ float sixth_exact(float h) {
+    constexpr double y = 1.0 / 6.0;
+    constexpr float yh = (float)y, yl = (float)(y - (double)(float)y);
+    bool sure = (fabsf(h) >= 0x1p-60f) & (fabsf(h) <= 0x1p+60f);
+    const float p = h * yh;
+    const float r = round_f2(F2{p, __fmaf_rn(h, yl, __fmaf_rn(h, yh, -p))}, sure);
+    return sure ? r : (float)(y * (double)h);
+}
+
+template <bool EXACT, class F, class A>
+__device__ __forceinline__ float3 step_rk4(const F& f, float3 p, float h, unsigned& ns, float3* b_raw, A& aside) {
     if constexpr (EXACT) {
         // the stages rolled (one sample in the loop body): the same
         // operations in the same order
         float3 q = p, sum = v3(0.f, 0.f, 0.f);
 #pragma unroll 1
         for (int st = 0; st < 4; ++st) {
+            aside(st);
             const float3 k = sample<true>(f, q, true);
             const float3 hk = h * k;
-            q = p + (st < 2 ? hk / 2.f : hk);
+            q = p + (st < 2 ? 0.5f * hk : hk);
             sum = st == 0 ? k : (st < 3 ? sum + 2.f * k : sum + k);
         }
         ns += 4;
-        return (float)(1.0 / 6.0 * (double)h) * sum;
+        return sixth_exact(h) * sum;
     }
     const float3 k1 = b_raw ? sample_unit_raw(f, p, *b_raw) : sample<EXACT>(f, p, true);
     const float3 k2 = sample<EXACT>(f, p + (h * k1) / 2.f, true);
@@ -296,7 +315,7 @@ __device__ __forceinline__ float3 step_rk4_normal(const F& f, float3 p, float h,
             k4 = k;
         }
     }
-    const float c = EXACT ? (float)(1.0 / 6.0 * (double)h) : h * (1.f / 6.f);
+    const float c = EXACT ? sixth_exact(h) : h * (1.f / 6.f);
     return p + c * (((k1 + 2.f * k2) + 2.f * k3) + k4);
 }
 
@@ -516,8 +535,11 @@ struct Lane {
     float h;       // current step
     float tol;     // local error tolerance (fast arithmetic: 0.2 log2(tol / 11.09), the controller's form)
     len_t len;     // accumulated length
-    float lc;      // Kahan compensation of len (fast arithmetic)
+    float lc;      // Kahan compensation of len (fast arithmetic); a float sum of the length (exact)
     double tw;     // accumulated twist
+    // exact arithmetic: the last step's length and twist integrand, not yet
+    // in len and tw (lane_pending)
+    float pend_dl, pend_td;
     int steps;     // accepted steps
     int rej;       // trial steps rejected in a row
     unsigned dsign;  // sign bit of the step: 0 forward, 0x80000000 backward
@@ -556,6 +578,8 @@ __device__ __forceinline__ void lane_begin(const F& f, const TraceJob<F>& J, Lan
     L.len = 0;
     L.lc = 0.f;
     L.tw = 0.0;
+    L.pend_dl = 0.f;
+    L.pend_td = 0.f;
     L.steps = 0;
     L.rej = 0;
     L.flag = 0;
@@ -595,13 +619,92 @@ __device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
     return d;
 }
 
+// The length limit; near: a float below which the float sum of the length
+// settles the exact arithmetic's comparison.
+template <bool EXACT>
+struct LenLimit {
+    typename Lane<EXACT>::len_t lim;
+    float near;
+};
+constexpr int kNearSteps = 100000;  // the float sum is then within 0.6 %
+
+// (double)td / 4 / pi in the reference's rounding: td / 4 is exact, the
+// quotient by pi comes from its reciprocal and once more from the exact
+// remainder (Markstein), that correction stretched and shrunk by 2^-20 to see
+// whether it could round otherwise (then the division).
+constexpr double kInvPi = 1.0 / kRefPi;
+__device__ __forceinline__ double over_4pi(float td, double u, double v) {
+    const bool sure = (u == v) & ((fabsf(td) >= 0x1p-100f) | (td == 0.f));
+    return sure ? u : (double)td / 4.0 / kRefPi;
+}
+
+// The exact twist kernels' per-step sums in double, one step behind: the
+// length's and the twist's FP64 operations (64 cycles each for a warp,
+// dependent on one another) run between the next step's samples instead of
+// on the way to it.  The same operations in the same order.  (Twist on 201 x
+// 203 x 4 seeds, curl included, 2.87 -> 2.72 ms; the length alone, in the
+// kernels without the twist, gains nothing: it is added at once.)
+struct Pending {
+    Lane<true>& L;
+    const bool tw_on;
+    double d, t, q, m, u, v;
+    __device__ __forceinline__ void operator()(int st) {
+        if (st == 0) {
+            d = (double)L.pend_dl;
+            if (tw_on) t = (double)(0.25f * L.pend_td);
+        } else if (st == 1) {
+            L.len = L.len + d;
+            if (tw_on) q = t * kInvPi;
+        } else if (st == 2) {
+            if (tw_on) m = __fma_rn(-q, kRefPi, t);
+        } else if (st == 3) {
+            if (tw_on) {
+                u = __fma_rn(m, kInvPi * (1.0 + 0x1p-20), q);
+                v = __fma_rn(m, kInvPi * (1.0 - 0x1p-20), q);
+            }
+        }
+    }
+    __device__ __forceinline__ void done() {
+        if (tw_on) {
+            L.tw = L.tw + over_4pi(L.pend_td, u, v) * d;
+            L.pend_td = 0.f;
+        }
+        L.pend_dl = 0.f;
+    }
+};
+// The pending step's sums at once; returns its twist increment.
+template <bool TWIST>
+__device__ __forceinline__ double lane_flush(Lane<true>& L, bool tw_on) {
+    const double d = (double)L.pend_dl;
+    L.len = L.len + d;
+    L.pend_dl = 0.f;
+    double dtw = 0.0;
+    if (TWIST && tw_on) {
+        dtw = (double)L.pend_td / 4.0 / kRefPi * d;
+        L.tw = L.tw + dtw;
+        L.pend_td = 0.f;
+    }
+    return dtw;
+}
+
 // The limits checked before a trial step: true (direction finished, L.out
 // and L.flag set) when the length or step limit stops it.
-template <bool EXACT, class F>
-__device__ __forceinline__ bool lane_limits(const TraceJob<F>& J, Lane<EXACT>& L,
-                                            typename Lane<EXACT>::len_t len_lim) {
+template <bool EXACT, bool TWIST, class F>
+__device__ __forceinline__ bool lane_limits(const TraceJob<F>& J, Lane<EXACT>& L, const LenLimit<EXACT>& limit,
+                                            bool tw_on) {
     const bool more_steps = EXACT ? ((long long)L.steps < J.prm.max_steps) : (L.steps < J.lim.max_steps);
-    const bool more_len = L.len < len_lim;
+    bool more_len;
+    if constexpr (EXACT) {
+        // the double comparison, and the wait for the last step's sum, only
+        // where the float sum does not settle it
+        more_len = (L.lc < limit.near) & (L.steps < kNearSteps);
+        if (!(more_len & more_steps)) {
+            lane_flush<TWIST>(L, tw_on);
+            more_len = L.len < limit.lim;
+        }
+    } else {
+        more_len = L.len < limit.lim;
+    }
     if (!(more_len & more_steps)) {
         L.out = L.p;
         L.flag = pack_flag(0, more_len ? QSL_LINE_MAX_STEPS : QSL_LINE_MAX_LENGTH);
@@ -702,16 +805,31 @@ __device__ __forceinline__ bool lane_move(const F& f, const TraceJob<F>& J, Lane
         p2 = v3(qxy.x, qxy.y, qz);
         dl = norm_fast(v3(txy.x, txy.y, tz));
     }
-    len_add(L, (double)dl, dl);
-    double dtw = 0.0;
-    if (TWIST && tw_on) {
-        dtw = EXACT ? (double)td / 4.0 / kRefPi * (double)dl : (double)(td * dl * kInv4PiF);
-        L.tw = L.tw + dtw;
-    }
     L.steps++;
-    if (!box_inside(f, p2)) {
-        len_add(L, -(double)dl, -dl);
-        if (TWIST && tw_on) L.tw = L.tw - dtw;
+    const bool left = !box_inside(f, p2);
+    if constexpr (EXACT) {
+        L.lc = L.lc + dl;
+        L.pend_dl = dl;
+        if (TWIST && tw_on) L.pend_td = td;
+        if (!TWIST && !left) lane_flush<TWIST>(L, tw_on);
+        if (left) {
+            const double dtw = lane_flush<TWIST>(L, tw_on);
+            L.len = L.len + -(double)dl;
+            if (TWIST && tw_on) L.tw = L.tw - dtw;
+        }
+    } else {
+        double dtw = 0.0;
+        len_add(L, 0.0, dl);
+        if (TWIST && tw_on) {
+            dtw = (double)(td * dl * kInv4PiF);
+            L.tw = L.tw + dtw;
+        }
+        if (left) {
+            len_add(L, 0.0, -dl);
+            if (TWIST && tw_on) L.tw = L.tw - dtw;
+        }
+    }
+    if (left) {
         L.out = p2;
         L.flag = kLaneExit;
         return true;
@@ -726,21 +844,31 @@ __device__ __forceinline__ bool lane_move(const F& f, const TraceJob<F>& J, Lane
 // TraceBline.cu:320-373.
 template <bool EXACT, bool TWIST, class F>
 __device__ __forceinline__ bool lane_step(const F& f, const TraceJob<F>& J, Lane<EXACT>& L,
-                                          typename Lane<EXACT>::len_t len_lim, bool tw_on,
-                                          unsigned& ns) {
-    if (lane_limits(J, L, len_lim)) return true;
+                                          const LenLimit<EXACT>& limit, bool tw_on, unsigned& ns) {
+    if (lane_limits<EXACT, TWIST>(J, L, limit, tw_on)) return true;
     const float hd = lane_hd(L);
     float3 inc;
     // fast twist kernels: B at L.p comes out of the step's first sample
     float3 b_at_p = v3(0.f, 0.f, 0.f);
     float3* const want_b = (!EXACT && TWIST && tw_on) ? &b_at_p : nullptr;
+    auto step = [&](auto& aside) {
+        float err = 0.f;
+        if (J.prm.integrator == QSL_RKF45) inc = step_rkf45<EXACT>(f, L.p, hd, err, ns, want_b, aside);
+        else inc = step_rk4<EXACT>(f, L.p, hd, ns, want_b, aside);
+        return err;
+    };
+    float err;
+    if constexpr (EXACT && TWIST) {
+        Pending pending{L, tw_on, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        err = step(pending);
+        pending.done();
+    } else {
+        Nothing nothing;
+        err = step(nothing);
+    }
     if (J.prm.integrator == QSL_RKF45) {
-        float err;
-        inc = step_rkf45<EXACT>(f, L.p, hd, err, ns, want_b);
         const int c = lane_control(J, L, err);
         if (c != 0) return c == 2;
-    } else {
-        inc = step_rk4<EXACT>(f, L.p, hd, ns, want_b);
     }
     return lane_move<EXACT, TWIST>(f, J, L, inc, b_at_p, tw_on, ns);
 }
@@ -805,6 +933,8 @@ __device__ __forceinline__ void lane_turn(const TraceJob<F>& J, Lane<EXACT>& L, 
     L.len = 0;
     L.lc = 0.f;
     L.tw = 0.0;
+    L.pend_dl = 0.f;
+    L.pend_td = 0.f;
     L.steps = 0;
     L.rej = 0;
     if (J.prm.integrator == QSL_RKF45) ns += 1;  // the tolerance's sample counts for both directions
@@ -933,7 +1063,7 @@ __device__ __forceinline__ unsigned lines_finish(const F& f, const TraceJob<F>& 
 // they are used rather than held in registers through the stepping loop.
 template <bool EXACT, bool TWIST, class F, class SL, class TC, class NR>
 __device__ __forceinline__ void trace_lines(const F& f, const TraceJob<F>& J, long long i, bool valid,
-                                            bool split, typename Lane<EXACT>::len_t len_lim, const SL& s_len_of,
+                                            bool split, const LenLimit<EXACT>& limit, const SL& s_len_of,
                                             const TC& tol_coef_of, const NR& nrm_of, bool tw_on, unsigned& ns) {
     Lane<EXACT> L;
     Stash<EXACT> S[2];
@@ -941,7 +1071,7 @@ __device__ __forceinline__ void trace_lines(const F& f, const TraceJob<F>& J, lo
         lane_begin<EXACT>(f, J, L, i, split && ((threadIdx.x >> 5) & 1) ? -1 : 1, s_len_of(), tol_coef_of(), nrm_of(),
                           ns);
         while (true) {
-            if (!lane_step<EXACT, TWIST>(f, J, L, len_lim, tw_on, ns)) continue;
+            if (!lane_step<EXACT, TWIST>(f, J, L, limit, tw_on, ns)) continue;
             stash_put<EXACT, TWIST>(S[L.dsign >> 31], L);
             if (split | (L.dsign != 0)) break;
             lane_turn(J, L, i, s_len_of(), ns);
@@ -1002,6 +1132,7 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
         len_lim = J.lim.len_lim;
     else
         len_lim = (typename Lane<EXACT>::len_t)(J.prm.len_ratio * len_scale(f));
+    const LenLimit<EXACT> limit{len_lim, 0.9f * (float)len_lim};
     unsigned ns = 0;
     const int lane_id = threadIdx.x & 31;
     const bool split = 2 * n_of() <= (long long)gridDim.x * blockDim.x;
@@ -1012,16 +1143,10 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
     if (queued) line = 0;
     while (true) {
         if (queued && line >= end) {
-            // lines per turn of the queue: the caller's choice, else an even
-            // share per warp of the grid between one warp's width (a small
-            // launch then uses every warp: with 256 the 128 x 128 plane ran
-            // on 64 of 2432 warps) and 256
-            long long chunk = J.chunk;
-            if (chunk <= 0) {
-                const long long warps = (long long)gridDim.x * (kTraceThreads / 32);
-                chunk = ((n_of() + warps - 1) / warps + 31) / 32 * 32;
-                chunk = chunk < 32 ? 32 : (chunk > 256 ? 256 : chunk);
-            }
+            // lines per turn of the queue: the caller's choice, else the
+            // warp's 32 (256 left the 128 x 128 plane on 64 of 2432 warps, 64
+            // a map of 131,072 seeds on 2048)
+            const long long chunk = J.chunk > 0 ? J.chunk : 32;
             unsigned long long base = 0;
             if (lane_id == 0) base = atomicAdd(J.queue, (unsigned long long)chunk);
             line = (long long)__shfl_sync(0xffffffffu, base, 0);
@@ -1030,7 +1155,7 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
         if (line >= n_of()) break;
         const bool valid = line + lane_id < (queued ? end : n_of());
         const long long i = (valid && J.order) ? (long long)__ldg(J.order + line + lane_id) : line + lane_id;
-        trace_lines<EXACT, TWIST>(f, J, i, valid, split, len_lim, s_len_of, tol_coef_of, nrm_of, tw_on, ns);
+        trace_lines<EXACT, TWIST>(f, J, i, valid, split, limit, s_len_of, tol_coef_of, nrm_of, tw_on, ns);
         // a lane's sample count nears 32 bits: hand it over (exact while one
         // line takes fewer than 5e8 trial steps)
         if (ns > (1u << 30)) {

@@ -1,7 +1,9 @@
 """The exact tracers' float forms of the reference's double arithmetic against
 the double arithmetic itself, bit for bit: the corner weights
-(weights_exact) at fractions of every kind a sample can have, and the step
-controller's power (step_scale_exact) at every float near its range."""
+(weights_exact) at fractions of every kind a sample can have, the step
+controller's power (step_scale_exact) at every float near its range, the
+offsets and quotients by constants, and a vector over its norm (unit_exact)
+against the IEEE square root and divisions."""
 import ctypes
 import subprocess
 
@@ -13,7 +15,7 @@ from fastqsl_gb300 import _build
 pytestmark = pytest.mark.gpu
 
 SOURCE = r"""
-#include "qsl_trace.cuh"
+#include "qsl_scott.cuh"
 using namespace qsl;
 __device__ bool same(float a, float b) { return a == b || (isnan(a) && isnan(b)); }
 __global__ void k_weights(const float* r, long long n, unsigned long long* bad) {
@@ -37,6 +39,37 @@ __global__ void k_scale(unsigned first, long long n, unsigned long long* bad) {
         const float q = __uint_as_float(first + (unsigned)i);
         if (!same(step_scale_exact(q), pow_cr((float)((double)q / 11.09), 0.2f))) atomicAdd(bad, 1ull);
     }
+}
+__global__ void k_unit(const float* r, long long n, unsigned long long* bad) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    for (long long i = t; i < n; i += step) {
+        const float x = r[3 * i], y = r[3 * i + 1], z = r[3 * i + 2];
+        const float nb = sqrtf(x * x + y * y + z * z);
+        const float3 u = unit_exact(v3(x, y, z));
+        if (!(same(u.x, x / nb) && same(u.y, y / nb) && same(u.z, z / nb))) atomicAdd(bad, 1ull);
+    }
+}
+__global__ void k_constants(const float* r, long long n, unsigned long long* bad) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    for (long long i = t; i < n; i += step) {
+        const float x = r[i];
+        bool ok = same(add_const_exact(x, PlusMilli{}), (float)((double)x + 0.001));
+        ok &= same(add_const_exact(x, MinusMilli{}), (float)((double)x - 0.001));
+        ok &= same(div_const_exact(x, 0.002f, 1.f / 0.002f), x / 0.002f);
+        ok &= same(sixth_exact(x), (float)(1.0 / 6.0 * (double)x));
+        const double td = (double)(0.25f * x), q = td * kInvPi, m = __fma_rn(-q, kRefPi, td);
+        const double w = over_4pi(x, __fma_rn(m, kInvPi * (1.0 + 0x1p-20), q), __fma_rn(m, kInvPi * (1.0 - 0x1p-20), q));
+        ok &= w == (double)x / 4.0 / kRefPi || isnan(w);
+        if (!ok) atomicAdd(bad, 1ull);
+    }
+}
+extern "C" int probe_unit(const float* r, long long n, unsigned long long* bad) {
+    k_unit<<<1216, 128>>>(r, n, bad);
+    return cudaDeviceSynchronize();
+}
+extern "C" int probe_constants(const float* r, long long n, unsigned long long* bad) {
+    k_constants<<<1216, 128>>>(r, n, bad);
+    return cudaDeviceSynchronize();
 }
 extern "C" int probe_weights(const float* r, long long n, unsigned long long* bad) {
     k_weights<<<1216, 128>>>(r, n, bad);
@@ -91,4 +124,46 @@ def test_exact_weights_equal_the_double_form(probe, kind):
 def test_exact_step_scale_equals_the_double_form(probe, first, count):
     bad = torch.zeros(1, dtype=torch.int64, device="cuda")
     assert probe.probe_scale(ctypes.c_uint(first), ctypes.c_longlong(count), ctypes.c_void_p(bad.data_ptr())) == 0
+    assert bad.item() == 0
+
+
+@pytest.mark.parametrize("kind", ["plain", "small", "uneven", "zeros", "extreme", "nodes"])
+def test_exact_unit_vector_equals_the_library(probe, kind):
+    n = 1 << 22
+    g = torch.Generator(device="cuda").manual_seed(13)
+    r = torch.randn(n, 3, generator=g, device="cuda")
+    e = torch.rand(n, 3, generator=g, device="cuda")
+    if kind == "small":
+        r = r * 1e-6
+    elif kind == "uneven":    # components far apart
+        r = r * torch.pow(10.0, -25.0 * e)
+    elif kind == "zeros":
+        r = torch.where(e < 0.4, 0.0, r)
+    elif kind == "extreme":   # squares that over- and underflow
+        r = r * torch.pow(10.0, 60.0 * e[:, :1] - 40.0)
+    elif kind == "nodes":     # few significant bits
+        r = torch.round(r * 8.0)
+    bad = torch.zeros(1, dtype=torch.int64, device="cuda")
+    assert probe.probe_unit(ctypes.c_void_p(r.contiguous().data_ptr()), ctypes.c_longlong(n),
+                            ctypes.c_void_p(bad.data_ptr())) == 0
+    assert bad.item() == 0
+
+
+@pytest.mark.parametrize("kind", ["coordinates", "near0", "powers", "all"])
+def test_exact_constants_equal_the_double_form(probe, kind):
+    n = 1 << 22
+    g = torch.Generator(device="cuda").manual_seed(17)
+    u = torch.rand(n, generator=g, device="cuda")
+    if kind == "coordinates":
+        x = 600.0 * u - 4.0
+    elif kind == "near0":
+        x = (u - 0.5) * 0.01
+    elif kind == "powers":
+        x = torch.round(u * 512.0) * torch.pow(2.0, -torch.floor(8.0 * torch.rand(n, generator=g, device="cuda")))
+    else:                     # every kind of float
+        x = torch.randint(-(1 << 31), (1 << 31) - 1, (n,), generator=g, device="cuda", dtype=torch.int64)
+        x = x.to(torch.int32).view(torch.float32)
+    bad = torch.zeros(1, dtype=torch.int64, device="cuda")
+    assert probe.probe_constants(ctypes.c_void_p(x.contiguous().data_ptr()), ctypes.c_longlong(n),
+                                 ctypes.c_void_p(bad.data_ptr())) == 0
     assert bad.item() == 0
