@@ -56,49 +56,67 @@ __device__ __forceinline__ float3 along(float3 u, const float3 g[3]) {
               dot(u, v3(g[0].z, g[1].z, g[2].z)));
 }
 
+struct PlusMilli {
+    static constexpr double value = 0.001;
+};
+
+// Exact arithmetic traces a line with eight lanes: the right-hand side's seven
+// samples (at p and at p +- 1e-3 e_j) are one lane's each, the rest of the
+// line's arithmetic is the same in all eight.  One lane to a line took the
+// samples one after the other in a kernel of 168-255 registers whose body
+// does not fit the instruction cache: a plane of 200 x 300 seeds in a 256 x
+// 256 x 128 box 2.35 -> 1.33 ms (1.69 with the seven samples in a rolled loop
+// of one lane).
+template <bool EXACT>
+constexpr int scott_lanes() { return EXACT ? 8 : 1; }
+__device__ __forceinline__ float3 oct_from(float3 v, int lane) {
+    const unsigned m = 0xffu << (threadIdx.x & 24);
+    return v3(__shfl_sync(m, v.x, lane), __shfl_sync(m, v.y, lane), __shfl_sync(m, v.z, lane));
+}
+
 // Unit field and its gradient by central differences of the unit field at
 // p +- 1e-3 e_j.  Exact arithmetic: the offset rounded as in double and
 // narrowed (as `x -= 0.001` on a float does), and the difference divided by
 // 0.002f.  Fast arithmetic: the offset 0.001f added in float and the
 // difference multiplied by 500 (rounding-level differences; no FP64 add or
 // IEEE divide, nine of each per right-hand side otherwise).
-struct PlusMilli {
-    static constexpr double value = 0.001;
-};
-struct MinusMilli {
-    static constexpr double value = -0.001;
-};
 template <bool EXACT, class F>
 __device__ __forceinline__ float3 unit_and_grad_fd(const F& f, float3 p, float3 g[3], unsigned& ns) {
+    ns += 7;
+    if constexpr (EXACT) {
+        const int base = threadIdx.x & 24, j = threadIdx.x & 7;
+        // lane 2 d + 1 samples below p on axis d, lane 2 d + 2 above, lanes 0
+        // and 7 at p; an offset below is the negated offset of the negated
+        // coordinate
+        const int d = (j - 1) >> 1;
+        float3 q = p;
+        if (j > 0 && j < 7) {
+            const float c = comp(p, d);
+            const float r = add_const_exact(j & 1 ? -c : c, PlusMilli{});
+            const float at = j & 1 ? -r : r;
+            if (d == 0) q.x = at;
+            else if (d == 1) q.y = at;
+            else q.z = at;
+        }
+        const float3 u = sample<true>(f, q, true);
+        const float3 db = u - oct_from(u, base + (j > 0 ? j - 1 : 0));
+        const float3 gj = v3(div_const_exact(db.x, 0.002f, 1.f / 0.002f), div_const_exact(db.y, 0.002f, 1.f / 0.002f),
+                             div_const_exact(db.z, 0.002f, 1.f / 0.002f));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) g[k] = oct_from(gj, base + 2 * k + 2);
+        return oct_from(u, base);
+    }
     const float3 b = sample<EXACT>(f, p, true);
-    // exact arithmetic: one axis per turn of a rolled loop (three samples in
-    // its body with b's instead of seven: unrolled, the right-hand side is
-    // fetched from beyond the instruction cache, 3.24 against 2.48 ms on a
-    // 200 x 300 plane in a 256 x 256 x 128 box)
-    constexpr int kTurns = EXACT ? 1 : 3;
-#pragma unroll kTurns
+#pragma unroll
     for (int j = 0; j < 3; ++j) {
         float3 lo = p, hi = p;
-        if (EXACT) {
-            const float c = comp(p, j);
-            const float a = add_const_exact(c, MinusMilli{}), b = add_const_exact(c, PlusMilli{});
-            if (j == 0) { lo.x = a; hi.x = b; }
-            if (j == 1) { lo.y = a; hi.y = b; }
-            if (j == 2) { lo.z = a; hi.z = b; }
-        } else {
-            if (j == 0) { lo.x = lo.x - 0.001f; hi.x = hi.x + 0.001f; }
-            if (j == 1) { lo.y = lo.y - 0.001f; hi.y = hi.y + 0.001f; }
-            if (j == 2) { lo.z = lo.z - 0.001f; hi.z = hi.z + 0.001f; }
-        }
+        if (j == 0) { lo.x = lo.x - 0.001f; hi.x = hi.x + 0.001f; }
+        if (j == 1) { lo.y = lo.y - 0.001f; hi.y = hi.y + 0.001f; }
+        if (j == 2) { lo.z = lo.z - 0.001f; hi.z = hi.z + 0.001f; }
         const float3 b1 = sample<EXACT>(f, lo, true);
         const float3 b2 = sample<EXACT>(f, hi, true);
-        const float3 db = b2 - b1;
-        if (EXACT)
-            g[j] = v3(div_const_exact(db.x, 0.002f, 1.f / 0.002f), div_const_exact(db.y, 0.002f, 1.f / 0.002f),
-                      div_const_exact(db.z, 0.002f, 1.f / 0.002f));
-        else g[j] = 500.f * db;
+        g[j] = 500.f * (b2 - b1);
     }
-    ns += 7;
     return b;
 }
 
@@ -262,9 +280,23 @@ __device__ void scott_line(const F& f, const ScottJob<F>& J, long long i, float 
     const qsl_trace_params& pr = J.prm;
     const ScottOut& o = J.o;
     const float3 p0 = v3(__ldg(J.inp_x + i), __ldg(J.inp_y + i), __ldg(J.inp_z + i));
-    const float3 bt = sample_endpoint<EXACT>(f, p0);
-    o.bthis_x[i] = bt.x; o.bthis_y[i] = bt.y; o.bthis_z[i] = bt.z;
+    // a line's lanes hold the same values: the first one writes them
+    const bool writes = scott_lanes<EXACT>() == 1 || (threadIdx.x & 7) == 0;
+    float3 bt;
+    if constexpr (EXACT) {
+        // a component per lane (the scalar interpolator runs in double)
+        const int k = threadIdx.x & 7, base = threadIdx.x & 24;
+        const float own = sample_scalar_exact(f, k < 2 ? k : 2, p0.x, p0.y, p0.z);
+        const unsigned m = 0xffu << base;
+        bt = v3(__shfl_sync(m, own, base), __shfl_sync(m, own, base + 1), __shfl_sync(m, own, base + 2));
+    } else {
+        bt = sample_endpoint<EXACT>(f, p0);
+    }
+    if (writes) {
+        o.bthis_x[i] = bt.x; o.bthis_y[i] = bt.y; o.bthis_z[i] = bt.z;
+    }
     if ((double)p0.z < -1e-8) {  // the reference skips seeds below z = 0
+        if (!writes) return;
         o.start_x[i] = 0.f; o.start_y[i] = 0.f; o.start_z[i] = 0.f; o.flag_start[i] = 0;
         o.end_x[i] = 0.f; o.end_y[i] = 0.f; o.end_z[i] = 0.f; o.flag_end[i] = 0;
         o.q0[i] = 0.f; o.qperp[i] = 0.f; o.line_len[i] = 0.0;
@@ -436,6 +468,7 @@ __device__ void scott_line(const F& f, const ScottJob<F>& J, long long i, float 
             qp = (float)(fabs(num) / (double)((nb0 * nb0) / (lBs * lBe)));
         }
     }
+    if (!writes) return;
     o.start_x[i] = es.p.x; o.start_y[i] = es.p.y; o.start_z[i] = es.p.z; o.flag_start[i] = fs;
     o.end_x[i] = ee.p.x; o.end_y[i] = ee.p.y; o.end_z[i] = ee.p.z; o.flag_end[i] = fe;
     o.q0[i] = q0;
@@ -445,7 +478,7 @@ __device__ void scott_line(const F& f, const ScottJob<F>& J, long long i, float 
 }
 
 // One line per thread (lockstep lanes on neighbouring seeds when J.order is
-// a tile order).
+// a tile order), or per eight threads (exact arithmetic).
 template <bool EXACT, int GRAD, bool TWIST, class F>
 __device__ __forceinline__ void scott_kernel_body(const ScottJob<F>& J) {
     F f = J.f;
@@ -460,14 +493,17 @@ __device__ __forceinline__ void scott_kernel_body(const ScottJob<F>& J) {
     long long n = J.s.n_dev ? (long long)__ldg(J.s.n_dev) : J.s.n;
     if (J.s.n_cap >= 0 && n > J.s.n_cap) n = J.s.n_cap;
     const bool tw_on = TWIST && (J.s.twist_flag_dev ? *J.s.twist_flag_dev : (J.s.twist_on != 0));
+    constexpr int kLanes = scott_lanes<EXACT>();
     unsigned ns = 0;
     unsigned long long ns_total = 0;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long line = (long long)blockIdx.x * blockDim.x + threadIdx.x; line < n; line += stride) {
+    const long long stride = (long long)gridDim.x * blockDim.x / kLanes;
+    for (long long line = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kLanes; line < n; line += stride) {
         const long long i = J.order ? (long long)__ldg(J.order + line) : line;
         scott_line<EXACT, GRAD, TWIST>(f, J, i, s_len, tol_coef, tw_on, ns);
-        ns_total += ns;
+        if (threadIdx.x % kLanes == 0) ns_total += ns;
         ns = 0;
+        // lanes of a line go on together (its shuffles name all eight)
+        if (kLanes > 1) __syncwarp(0xffu << (threadIdx.x & 24));
     }
     if (J.samples) {
         __syncwarp();

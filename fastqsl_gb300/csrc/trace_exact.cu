@@ -48,8 +48,10 @@ cudaError_t launch_trace_exact_stretch_uni(const TraceJob<FieldStretchU>& J, boo
     return launch_exact(J, twist, sched, n_host, st);
 }
 
+// (5 blocks per SM: 1.33 ms on the plane of qsl_scott.cuh's figures, 1.80 with
+// the compiler's 208 registers)
 template <bool TWIST>
-__global__ void __launch_bounds__(kTraceBlock) k_scott_exact(const ScottJob<FieldSoA> J) {
+__global__ void __launch_bounds__(kTraceBlock, 5) k_scott_exact(const ScottJob<FieldSoA> J) {
     scott_kernel_body<true, GRAD_FD, TWIST>(J);
 }
 
@@ -59,7 +61,7 @@ static int grid_for_lines(long long n) {
 }
 
 cudaError_t launch_scott_exact(const ScottJob<FieldSoA>& J, bool twist, long long n_grid, cudaStream_t st) {
-    const int grid = grid_for_lines(n_grid);
+    const int grid = grid_for_lines(n_grid * scott_lanes<true>());
     if (twist) k_scott_exact<true><<<grid, kTraceBlock, 0, st>>>(J);
     else k_scott_exact<false><<<grid, kTraceBlock, 0, st>>>(J);
     return cudaGetLastError();

@@ -54,7 +54,7 @@ __global__ void k_constants(const float* r, long long n, unsigned long long* bad
     for (long long i = t; i < n; i += step) {
         const float x = r[i];
         bool ok = same(add_const_exact(x, PlusMilli{}), (float)((double)x + 0.001));
-        ok &= same(add_const_exact(x, MinusMilli{}), (float)((double)x - 0.001));
+        ok &= same(-add_const_exact(-x, PlusMilli{}), (float)((double)x - 0.001));
         ok &= same(div_const_exact(x, 0.002f, 1.f / 0.002f), x / 0.002f);
         ok &= same(sixth_exact(x), (float)(1.0 / 6.0 * (double)x));
         const double td = (double)(0.25f * x), q = td * kInvPi, m = __fma_rn(-q, kRefPi, td);
