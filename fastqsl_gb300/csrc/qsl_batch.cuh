@@ -11,18 +11,52 @@
 
 namespace qsl {
 
+// The lines of one job that a warp holds: the first of them, counted from the
+// job's start, and how the warp shares them (trace_lines, spread_of).
+struct BatchSlot {
+    long long first;
+    bool split;
+    int spread;
+};
+
+// The lines of one warp's turn in a job whose range starts at `begin` and
+// holds `room` lines; `g` is the warp's line in the launch's line space.
+//
+// A job whose count comes from the device (n_dev) usually fills a small part
+// of its range, and the warps past it would start and exit.  When the whole
+// batch runs in one launch, its lines go to all the job's warps: directions
+// to pairs of warps and up to four lanes per line, as in a launch of their
+// own (all after the main trace of two requests
+// of 17,000 seeds: 0.90 -> 0.75 ms).
+template <class F>
+__device__ __forceinline__ BatchSlot batch_slot(const TraceJob<F>& J, long long n, long long g, long long begin,
+                                                long long room, bool whole) {
+    if (J.s.n_dev && whole) {
+        // the job's warps as pairs of the block; its first warp may be the
+        // second of a pair
+        const long long warp = (g - begin) / 32;
+        const int odd = (int)(((threadIdx.x >> 5) ^ (unsigned)warp) & 1u);
+        const long long usable = (room / 32 - odd) & ~1LL;
+        if (splits(n, usable)) {
+            int s = spread_of(n, usable);
+            while (s > 1 && 2 * ((n * s + 31) / 32) > usable) s /= 2;
+            if (2 * ((n * s + 31) / 32) <= usable)
+                return {warp < odd ? n : ((warp - odd) >> 1) * (32 / s), true, s};
+        }
+    }
+    return {g - begin, false, 1};
+}
+
 template <bool TWIST, class F>
-__device__ __forceinline__ void batch_line(const TraceJob<F>& J, long long line, bool in_window,
-                                           bool split, unsigned& ns) {
+__device__ __forceinline__ void batch_line(const TraceJob<F>& J, const BatchSlot& slot, long long n, long long left,
+                                           unsigned& ns) {
     F f = J.f;
     if (f.d.nx < 2 || f.d.ny < 2 || f.d.nz < 2) return;
-    long long n = J.s.n;
-    if (J.s.n_dev) {  // count produced on the device; the range was sized by n
-        const long long nd = (long long)__ldg(J.s.n_dev);
-        n = nd < n ? nd : n;
-    }
-    if (line - (threadIdx.x & 31) >= n) return;  // past the job's lines (a whole warp, or a whole pair)
-    const bool valid = in_window && line < n;    // else a padding lane of the job's warp-aligned range
+    const int lane = threadIdx.x & 31;
+    const long long line = slot.first + lane / slot.spread;
+    if (slot.first >= n) return;  // past the job's lines (a whole warp, or a whole pair)
+    // else lanes past the job's lines or the window, or between spread lines
+    const bool valid = lane % slot.spread == 0 && line < n && lane / slot.spread < left;
     const long long i = (valid && J.order) ? (long long)__ldg(J.order + line) : line;
     const bool tw_on = TWIST && J.s.twist_on != 0;
     store_prepare(f);
@@ -33,8 +67,8 @@ __device__ __forceinline__ void batch_line(const TraceJob<F>& J, long long line,
     else
         len_lim = (float)(J.prm.len_ratio * len_scale(f));
     trace_lines<false, TWIST>(
-        f, J, i, valid, split, LenLimit<false>{len_lim, 0.f}, [&J]() { return J.s.s_len; }, [&J]() { return J.s.tol_coef; },
-        [&J]() { return v3(J.s.cross[0], J.s.cross[1], J.s.cross[2]); }, tw_on, ns);
+        f, J, i, valid, slot.split, LenLimit<false>{len_lim, 0.f}, [&J]() { return J.s.s_len; },
+        [&J]() { return J.s.tol_coef; }, [&J]() { return v3(J.s.cross[0], J.s.cross[1], J.s.cross[2]); }, tw_on, ns);
 }
 
 // begin[j]: first line of job j (multiples of 32, increasing); begin[njobs]:
@@ -47,23 +81,34 @@ __device__ __forceinline__ void batch_kernel_body(const TraceJob<F>* __restrict_
                                                   unsigned long long* samples, long long line_lo,
                                                   long long line_hi) {
     long long total = __ldg(begin + njobs);
+    const bool whole = line_lo == 0 && line_hi >= total;
     total = line_hi < total ? line_hi : total;
-    const int lane = threadIdx.x & 31;
-    const long long threads = (long long)gridDim.x * blockDim.x;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane;
-    // two threads per line: the directions over warp pairs (trace_lines)
-    const bool split = 2 * (total - line_lo) <= threads;
-    const long long stride = split ? threads / 2 : threads;
+    const long long warps = (long long)gridDim.x * (kTraceThreads / 32);
+    const long long w = (long long)blockIdx.x * (kTraceThreads / 32) + (threadIdx.x >> 5);
+    // lanes to spare: the directions over warp pairs, fewer lines per warp
+    const bool split = splits(total - line_lo, warps);
+    const int spread = split ? spread_of(total - line_lo, warps) : 1;
+    const int lines = 32 / spread;
+    const long long stride = warps * lines / (split ? 2 : 1);
     unsigned ns = 0;
     unsigned long long ns_total = 0;
-    for (long long g = line_lo + (split ? (t >> 6) * 32 : t); g < total; g += stride) {
+    for (long long g = line_lo + (split ? w >> 1 : w) * lines; g < total; g += stride) {
         int lo = 0, hi = njobs - 1;  // last j with begin[j] <= g
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
             if (__ldg(begin + mid) <= g) lo = mid;
             else hi = mid - 1;
         }
-        batch_line<TWIST>(jobs[lo], g + lane - __ldg(begin + lo), g + lane < total, split, ns);
+        const TraceJob<F>& J = jobs[lo];
+        const long long b = __ldg(begin + lo);
+        long long n = J.s.n;
+        if (J.s.n_dev) {  // count produced on the device; the range was sized by n
+            const long long nd = (long long)__ldg(J.s.n_dev);
+            n = nd < n ? nd : n;
+        }
+        const BatchSlot slot =
+            split ? BatchSlot{g - b, true, spread} : batch_slot(J, n, g, b, __ldg(begin + lo + 1) - b, whole);
+        batch_line<TWIST>(J, slot, n, split | !slot.split ? total - g : 32, ns);
         ns_total += ns;
         ns = 0;
     }

@@ -19,14 +19,19 @@ constexpr int kTraceBlock = kTraceThreads;
 // count: the persistent grid.
 int persistent_grid(const void* kernel, int block, size_t smem = 0);
 
-// Grid of a static tracer launch of n lines, for a kernel of which
-// `resident` blocks fit on the GPU at a time: two warps per 32 lines, one per
-// direction (trace_lines' split), where all of them are resident together,
-// else one thread per line.
+// Grid of a static tracer launch of n lines, for a kernel of which `resident`
+// blocks fit on the GPU at a time: two warps per warp's worth of lines, one
+// per direction, and up to kMaxSpread lanes per line, as far as all of them
+// are resident together; else one thread per line.
 inline int static_grid(long long n, int resident) {
-    const long long pairs = 64 * ((n + 31) / 32);
-    long long g = pairs <= (long long)resident * kTraceBlock ? pairs : n;
-    g = (g + kTraceBlock - 1) / kTraceBlock;
+    const long long warps = (long long)resident * (kTraceBlock / 32);
+    long long threads = n;
+    if (splits(n + 31, warps)) {
+        int s = spread_of(n, warps);
+        while (s > 1 && 2 * ((n * s + 31) / 32) > warps) s /= 2;
+        threads = 64 * ((n * s + 31) / 32);
+    }
+    const long long g = (threads + kTraceBlock - 1) / kTraceBlock;
     return (int)(g < 1 ? 1 : (g > (1 << 30) ? (1 << 30) : g));
 }
 
