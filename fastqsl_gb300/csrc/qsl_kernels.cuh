@@ -14,6 +14,20 @@ __global__ void __launch_bounds__(kTraceBlock, MINB) k_trace_fast(const __grid_c
     trace_kernel_body<false, TWIST, QUEUE>(J);
 }
 
+// The static brick kernel in blocks of 256, for launches of many waves: four
+// 8 x 8 seed tiles then share an SM's L1 instead of two (258 x 258 x 128 seeds
+// of a 512 x 512 x 256 field 106.1 -> 103.4 ms).  Launches of a wave or two
+// lose by it (258 x 514 seeds 1.14 -> 1.18 ms: a block's warps wait for its
+// longest line), and below a full wave the directions split over pairs of
+// warps, which the 128-thread blocks are made for.
+constexpr int kWideBlock = 256;
+constexpr int kWideWaves = 8;
+template <bool TWIST, class F, int MINB>
+__global__ void __launch_bounds__(kWideBlock, MINB* kTraceBlock / kWideBlock)
+    k_trace_fast_wide(const __grid_constant__ TraceJob<F> J) {
+    trace_kernel_body<false, TWIST, false>(J);
+}
+
 template <class F, int MINB>
 static cudaError_t launch_fast_minb(const TraceJob<F>& J, bool twist, Schedule sched, long long n_host,
                                     cudaStream_t st) {
@@ -29,6 +43,14 @@ static cudaError_t launch_fast_minb(const TraceJob<F>& J, bool twist, Schedule s
         // over the whole capacity whose surplus blocks would each start and
         // exit
         const int waves = 2 * grid;
+        if constexpr (std::is_same<F, FieldH4B>::value && MINB == 6) {
+            const long long blocks = (n_host + kWideBlock - 1) / kWideBlock;
+            if (grid > 0 && !J.s.n_dev && n_host >= (long long)kWideWaves * grid * kTraceBlock && blocks <= (1 << 30)) {
+                if (twist) k_trace_fast_wide<true, F, MINB><<<(int)blocks, kWideBlock, 0, st>>>(J);
+                else k_trace_fast_wide<false, F, MINB><<<(int)blocks, kWideBlock, 0, st>>>(J);
+                return cudaGetLastError();
+            }
+        }
         grid = static_grid(n_host, grid);
         if (J.s.n_dev && waves > 0 && grid > waves) grid = waves;
     }

@@ -28,7 +28,7 @@
 
 namespace qsl {
 
-constexpr int kTraceThreads = 128;  // threads per block of every tracer kernel
+constexpr int kTraceThreads = 128;  // threads per block of the tracer kernels (kWideBlock in one case)
 
 constexpr double kRefPi = 3.14159265;  // the reference's M_PI (TraceBlineAdaptive.cu:10)
 // 1 / (4 pi) for the fast twist increment: one float product per step and a
@@ -1182,13 +1182,13 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
     const LenLimit<EXACT> limit{len_lim, 0.9f * (float)len_lim};
     unsigned ns = 0;
     const int lane_id = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (kTraceThreads / 32);
+    const long long warps = (long long)gridDim.x * (blockDim.x / 32);
     const bool split = splits(n_of(), warps);
     const int spread = split ? spread_of(n_of(), warps) : 1;
     const int lines = 32 / spread;  // of a warp
     const bool queued = QUEUE && !split;
     // the warp's first line, and the end of its chunk
-    long long line = (long long)blockIdx.x * (kTraceThreads / 32) + (threadIdx.x >> 5), end = 0;
+    long long line = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), end = 0;
     line = queued ? 0 : (split ? line >> 1 : line) * lines;
     while (true) {
         if (queued && line >= end) {

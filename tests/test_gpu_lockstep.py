@@ -82,3 +82,19 @@ def test_batch_equals_one_launch(field, seeds, n):
     plan.launch()
     for k, v in whole.items():
         assert torch.equal(out[k], v) or np.array_equal(out[k].cpu().numpy(), v.cpu().numpy(), equal_nan=True), k
+
+
+@pytest.mark.parametrize("twist", [False, True])
+def test_wide_blocks_equal_narrow_ones(field, twist):
+    """Launches of many waves on bricks run in blocks of 256 threads at the
+    6-block budget; the 7-block budget keeps blocks of 128."""
+    from fastqsl_gb300 import api
+    n = 1200037  # over 8 waves of 6 x 128 threads on every SM, last warp partly filled
+    g = torch.Generator(device="cuda").manual_seed(8)
+    s = [(63.0 * torch.rand(n, generator=g, device="cuda")).contiguous() for _ in range(3)]
+    store = api.FieldStore(*field, layout="h4b")
+    cur = [api.as_xfast(b.roll(1, 0).contiguous()) for b in field] if twist else None
+    prm = P.absolute_rkf45(tol=1e-2)
+    a, b = (api.trace(store, *s, prm, s_len=0.5, curB=cur, schedule="static", occupancy=k) for k in (6, 7))
+    for k, v in a.items():
+        assert v is None or np.array_equal(v.cpu().numpy(), b[k].cpu().numpy(), equal_nan=v.is_floating_point()), k
