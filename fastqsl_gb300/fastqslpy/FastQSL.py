@@ -83,34 +83,35 @@ def CookPseudoLine(x_end_arr, y_end_arr, z_end_arr, flag_end_arr,
     dev = bf.device
     n = int(bf.numel())
     lib = _lib.load()
-    cut = [torch.empty(4 * n, dtype=torch.float32, device=dev) for _ in range(3)]
-    bz0s = torch.empty(n, dtype=torch.float32, device=dev)
-    bz0e = torch.empty(n, dtype=torch.float32, device=dev)
+    # arrays of a kind as rows of one allocation (a zeroing or a copy is then
+    # one launch for all of them; each row is contiguous)
+    cut = torch.empty((3, 4 * n), dtype=torch.float32, device=dev)
+    bz0 = torch.empty((2, n), dtype=torch.float32, device=dev)
     count = torch.zeros(2, dtype=torch.int64, device=dev)
     wb = int(lib.qsl_cook_workspace_bytes(n))
     work = torch.empty((wb + 7) // 8, dtype=torch.int64, device=dev)
     _lib.check(lib.qsl_cook_pseudo_line(ptr(bf), ptr(_t(x_start_arr)), ptr(_t(y_start_arr)), ptr(_t(z_start_arr)),
                                         ptr(_t(flag_start_arr)), ptr(_t(Bz_in_arr)), ptr(_t(Bz_out_arr)), n, 1, n, 0,
                                         float(np.float32(stride_this)), ptr(cut[0]), ptr(cut[1]), ptr(cut[2]),
-                                        ptr(bz0s), ptr(bz0e), None, ptr(count), ptr(work), wb, stream_handle()),
+                                        ptr(bz0[0]), ptr(bz0[1]), None, ptr(count), ptr(work), wb, stream_handle()),
                "CookPseudoLine")
     k = int(count[0].item())
     m = 4 * k
-    cut_inp_x, cut_inp_y, cut_inp_z = (c[:m].clone() for c in cut)
-    z = [torch.zeros(m, dtype=torch.float32, device=dev) for _ in range(15)]
+    cut_inp_x, cut_inp_y, cut_inp_z = cut[:, :m].clone(memory_format=torch.contiguous_format).unbind(0)
+    Bz0_start, Bz0_end = bz0[:, :k].clone(memory_format=torch.contiguous_format).unbind(0)
     (cut_start_x, cut_start_y, cut_start_z, cut_end_x, cut_end_y, cut_end_z,
      Bx_start_cut, By_start_cut, Bz_start_cut, Bx_end_cut, By_end_cut, Bz_end_cut,
-     Bx_inp_cut, By_inp_cut, Bz_inp_cut) = z
+     Bx_inp_cut, By_inp_cut, Bz_inp_cut) = torch.zeros((15, m), dtype=torch.float32, device=dev).unbind(0)
     line_len_cut = torch.zeros(m, dtype=torch.float64, device=dev)
     N_cut = _uint64(m, dev)
-    B_flag_cut, flag_cut_start, flag_cut_end = (torch.zeros(m, dtype=torch.int32, device=dev) for _ in range(3))
+    B_flag_cut, flag_cut_start, flag_cut_end = torch.zeros((3, m), dtype=torch.int32, device=dev).unbind(0)
     return (cut_inp_x, cut_inp_y, cut_inp_z,
             cut_start_x, cut_start_y, cut_start_z, flag_cut_start,
             cut_end_x, cut_end_y, cut_end_z, flag_cut_end,
             Bx_inp_cut, By_inp_cut, Bz_inp_cut, B_flag_cut,
             Bx_start_cut, By_start_cut, Bz_start_cut,
             Bx_end_cut, By_end_cut, Bz_end_cut, N_cut, line_len_cut,
-            bz0s[:k].clone(), bz0e[:k].clone())
+            Bz0_start, Bz0_end)
 
 
 def QCalcCut(cut_start_x, cut_start_y, cut_start_z, flag_cut_start,

@@ -19,7 +19,8 @@ _ARITH = {"exact": 0, "fast": 1}
 
 def _current_stream(args):
     for a in args:
-        if hasattr(a, "__cuda_array_interface__") and not hasattr(a, "data_ptr"):
+        # (a tensor builds its __cuda_array_interface__ anew at every look)
+        if not hasattr(a, "data_ptr") and hasattr(a, "__cuda_array_interface__"):
             try:
                 import cupy  # the caller's arrays are CuPy: use CuPy's current stream
                 return cupy.cuda.get_current_stream().ptr
