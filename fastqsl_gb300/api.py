@@ -565,14 +565,13 @@ class QMapPlan:
             qdone = torch.cuda.Event()
             qdone.record(self._side)
         s = self.sub
-        _lib.check(lib.qsl_qcut(ptr(s["start_x"]), ptr(s["start_y"]), ptr(s["start_z"]), ptr(s["flag_start"]),
-                                ptr(s["end_x"]), ptr(s["end_y"]), ptr(s["end_z"]), ptr(s["flag_end"]),
-                                ptr(self.bz0s), ptr(self.bz0e), 0, ptr(self.count[0:1]), self.max_pix, jac, None,
-                                ptr(self.qcut), st), "qsl_qcut")
         if overlap:
             ev_stream.wait_event(qdone)
-        _lib.check(lib.qsl_qmerge(ptr(self.pix), None, ptr(self.qcut), 0, ptr(self.count[0:1]), self.max_pix,
-                                  self.n0, self.n1, None, ptr(self.Q), st), "qsl_qmerge")
+        _lib.check(lib.qsl_qcut_merge(ptr(s["start_x"]), ptr(s["start_y"]), ptr(s["start_z"]), ptr(s["flag_start"]),
+                                      ptr(s["end_x"]), ptr(s["end_y"]), ptr(s["end_z"]), ptr(s["flag_end"]),
+                                      ptr(self.bz0s), ptr(self.bz0e), 0, ptr(self.count[0:1]), self.max_pix, jac,
+                                      ptr(self.pix), self.n0, self.n1, ptr(self.qcut), ptr(self.Q), st),
+                   "qsl_qcut_merge")
         return self.Q
 
 
@@ -947,12 +946,11 @@ class QBatch:
         for J in self.jobs:
             sp, s = J["sp"], J["sub"]
             jac = (1.0 / (2.0 * float(sp.get("stride", 1.0)))) ** 4.0
-            _lib.check(lib.qsl_qcut(ptr(s["start_x"]), ptr(s["start_y"]), ptr(s["start_z"]), ptr(s["flag_start"]),
-                                    ptr(s["end_x"]), ptr(s["end_y"]), ptr(s["end_z"]), ptr(s["flag_end"]),
-                                    ptr(J["bz0s"]), ptr(J["bz0e"]), 0, J["count"], J["m"], jac, None,
-                                    ptr(J["qcut"]), st), "qcut")
-            _lib.check(lib.qsl_qmerge(ptr(J["pix"]), None, ptr(J["qcut"]), 0, J["count"], J["m"],
-                                      J["n0"], J["n1"], None, ptr(J["Q"]), st), "qmerge")
+            _lib.check(lib.qsl_qcut_merge(ptr(s["start_x"]), ptr(s["start_y"]), ptr(s["start_z"]),
+                                          ptr(s["flag_start"]), ptr(s["end_x"]), ptr(s["end_y"]), ptr(s["end_z"]),
+                                          ptr(s["flag_end"]), ptr(J["bz0s"]), ptr(J["bz0e"]), 0, J["count"], J["m"],
+                                          jac, ptr(J["pix"]), J["n0"], J["n1"], ptr(J["qcut"]), ptr(J["Q"]), st),
+                       "qcut_merge")
         return [J["Q"] for J in self.jobs]
 
     def capture(self):

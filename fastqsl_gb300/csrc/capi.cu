@@ -1170,6 +1170,27 @@ int qsl_qcut(const float* start_x, const float* start_y, const float* start_z, c
     return QSL_OK;
 }
 
+int qsl_qcut_merge(const float* start_x, const float* start_y, const float* start_z, const int* flag_start,
+                   const float* end_x, const float* end_y, const float* end_z, const int* flag_end,
+                   const float* Bz0_start, const float* Bz0_end, int64_t count, const unsigned long long* count_dev,
+                   int64_t max_count, double jac_scale, const int64_t* pix, int n0, int n1, double* Qcut64,
+                   double* Qfinal64, qsl_stream_t stream) {
+    if (!start_x || !start_y || !start_z || !flag_start || !end_x || !end_y || !end_z || !flag_end ||
+        !Bz0_start || !Bz0_end || !pix || !Qcut64 || !Qfinal64)
+        return fail(QSL_ERR_INVALID, "null pointer");
+    if (n0 < 3 || n1 < 3) return fail(QSL_ERR_INVALID, "plane must be at least 3 x 3");
+    QcutArgs a;
+    a.xs = start_x; a.ys = start_y; a.zs = start_z; a.fs = flag_start;
+    a.xe = end_x; a.ye = end_y; a.ze = end_z; a.fe = flag_end;
+    a.bz0s = Bz0_start; a.bz0e = Bz0_end;
+    a.count_dev = count_dev; a.count = count;
+    a.k32 = (float)jac_scale; a.k64 = jac_scale;
+    a.q32 = nullptr; a.q64 = Qcut64;
+    QSL_CHECK_CUDA(launch_qcut_merge(a, count_dev ? max_count : count, (const long long*)pix, n0, n1, Qfinal64,
+                                     (cudaStream_t)stream), "qcut_merge");
+    return QSL_OK;
+}
+
 int qsl_qmerge(const int64_t* pix, const float* Qcut32, const double* Qcut64, int64_t count,
                const unsigned long long* count_dev, int64_t max_count, int n0, int n1, float* Qfinal32,
                double* Qfinal64, qsl_stream_t stream) {

@@ -177,9 +177,40 @@ __global__ void __launch_bounds__(1024) k_tile_scan(const int* tile_count, long 
 }
 
 
+// The sum of a block of kTile threads' values, in every thread.
+__device__ __forceinline__ int block_sum(int v) {
+    __shared__ int part[kTile / 32];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = part[threadIdx.x & 31];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Tiles up to which a tile's block sums the counts before it itself (one per
+// thread) instead of reading a scan kernel's offsets: one launch less between
+// the main trace and the pseudo-line trace, ~5 us of a 100 x 100 map's 230.
+constexpr long long kSelfScan = kTile;
+
 // The selected pixels of one tile and their pseudo-line seeds, written in
-// pixel order by a block of kTile threads.
-__device__ __forceinline__ void cook_write_tile(const CookArgs& a, long long tile) {
+// pixel order by a block of kTile threads.  SCAN: the block forms its offset
+// from the counts (ntiles <= kSelfScan) and the last tile's writes the totals;
+// else both come from k_tile_scan.
+template <bool SCAN>
+__device__ __forceinline__ void cook_write_tile(const CookArgs& a, long long tile, long long ntiles,
+                                                const int* tile_count, unsigned long long* total) {
+    long long off;
+    if (SCAN) {
+        off = block_sum(threadIdx.x < tile ? tile_count[threadIdx.x] : 0);
+        if (tile == ntiles - 1 && threadIdx.x == 0) {
+            const unsigned long long t = (unsigned long long)(off + tile_count[tile]);
+            total[0] = t;      // selected pixels
+            total[1] = 4 * t;  // their pseudo-line seeds
+        }
+    } else {
+        off = a.tile_off[tile];
+    }
     const long long p = tile * kTile + threadIdx.x;
     const bool sel = p < a.n && pixel_selected(a.bflag, p, a.n0, a.n1, a.interior_only);
     __shared__ int wcount[kTile / 32];
@@ -192,7 +223,7 @@ __device__ __forceinline__ void cook_write_tile(const CookArgs& a, long long til
     for (int w = 0; w < warp; ++w) before += wcount[w];
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-    const long long k = a.tile_off[tile] + before + __popc(m & lt);
+    const long long k = off + before + __popc(m & lt);
     const float x = a.xs[p], y = a.ys[p], z = a.zs[p];
     const int f = a.fs[p];
     const int d = (f >= 1 && f <= 6) ? (f - 1) / 2 : -1;
@@ -212,11 +243,29 @@ __device__ __forceinline__ void cook_write_tile(const CookArgs& a, long long til
     if (a.pix) a.pix[k] = p;
 }
 
-__global__ void __launch_bounds__(kTile) k_cook_write(const CookArgs a) { cook_write_tile(a, blockIdx.x); }
+template <bool SCAN>
+__global__ void __launch_bounds__(kTile) k_cook_write(const CookArgs a, const int* tile_count,
+                                                      unsigned long long* total) {
+    cook_write_tile<SCAN>(a, blockIdx.x, gridDim.x, tile_count, total);
+}
 
+// Where the merge writes a pixel's Q at once (qmap null: it does not).
+struct QcutMerge {
+    const long long* pix;
+    int n0, n1;
+    double* qmap;
+};
+template <class TQ>
+__device__ __forceinline__ void merge_pixel(long long p, TQ q, int n0, int n1, TQ* qfinal) {
+    const long long per = (long long)n0 * n1, per2 = (long long)(n0 - 2) * (n1 - 2);
+    const long long pl = p / per, r = p % per;
+    const int i = (int)(r / n1), j = (int)(r % n1);
+    if (i >= 1 && i <= n0 - 2 && j >= 1 && j <= n1 - 2)
+        qfinal[pl * per2 + (long long)(i - 1) * (n1 - 2) + (j - 1)] = q;
+}
 
 template <bool F64>
-__device__ __forceinline__ void qcut_range(const QcutArgs& a, long long first, long long stride) {
+__device__ __forceinline__ void qcut_range(const QcutArgs& a, const QcutMerge& M, long long first, long long stride) {
     typedef typename std::conditional<F64, double, float>::type T;
     const long long cnt = a.count_dev ? (long long)*a.count_dev : a.count;
     for (long long k = first; k < cnt; k += stride) {
@@ -242,26 +291,20 @@ __device__ __forceinline__ void qcut_range(const QcutArgs& a, long long first, l
         if (q < (T)1) q = (T)1;
         if (F64) a.q64[k] = (double)q;
         else a.q32[k] = (float)q;
+        if (F64 && M.qmap) merge_pixel(M.pix[k], (double)q, M.n0, M.n1, M.qmap);
     }
 }
 
 template <bool F64>
-__global__ void k_qcut(const QcutArgs a) {
-    qcut_range<F64>(a, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+__global__ void k_qcut(const QcutArgs a, const QcutMerge M) {
+    qcut_range<F64>(a, M, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
 // Q_final[plane, i-1, j-1] = Qcut[k] for each compacted interior pixel.
 template <class TQ, class TC>
 __device__ __forceinline__ void qmerge_range(const long long* pix, const TC* qcut, long long cnt, int n0, int n1,
                                              TQ* qfinal, long long first, long long stride) {
-    const long long per = (long long)n0 * n1, per2 = (long long)(n0 - 2) * (n1 - 2);
-    for (long long k = first; k < cnt; k += stride) {
-        const long long p = pix[k];
-        const long long pl = p / per, r = p % per;
-        const int i = (int)(r / n1), j = (int)(r % n1);
-        if (i >= 1 && i <= n0 - 2 && j >= 1 && j <= n1 - 2)
-            qfinal[pl * per2 + (long long)(i - 1) * (n1 - 2) + (j - 1)] = (TQ)qcut[k];
-    }
+    for (long long k = first; k < cnt; k += stride) merge_pixel(pix[k], (TQ)qcut[k], n0, n1, qfinal);
 }
 
 template <class TQ, class TC>
@@ -307,30 +350,23 @@ __global__ void __launch_bounds__(1024) k_tile_scan_jobs(const QPostJob* jobs, c
     tile_scan_block(jobs[j].tile_count, tb[j + 1] - tb[j], jobs[j].tile_off, jobs[j].total);
 }
 
+template <bool SCAN>
 __global__ void __launch_bounds__(kTile) k_cook_write_jobs(const QPostJob* jobs, const long long* begin, int njobs) {
     const long long* tb = begin + (njobs + 1);
     const long long b = blockIdx.x;
     const int j = post_job(tb, njobs, b);
     const CookArgs a = jobs[j].c;
-    cook_write_tile(a, b - tb[j]);
+    cook_write_tile<SCAN>(a, b - tb[j], tb[j + 1] - tb[j], jobs[j].tile_count, jobs[j].total);
 }
 
 __global__ void __launch_bounds__(256) k_qcut_jobs(const QPostJob* jobs, const long long* begin, int njobs) {
     const long long* cb = begin + 2 * (njobs + 1);
     const long long b = blockIdx.x;
     const int j = post_job(cb, njobs, b);
-    const QcutArgs a = jobs[j].k;
-    qcut_range<true>(a, (b - cb[j]) * blockDim.x + threadIdx.x, jobs[j].cblocks * blockDim.x);
-}
-
-__global__ void __launch_bounds__(256) k_qmerge_jobs(const QPostJob* jobs, const long long* begin, int njobs) {
-    const long long* cb = begin + 2 * (njobs + 1);
-    const long long b = blockIdx.x;
-    const int j = post_job(cb, njobs, b);
     const QPostJob& J = jobs[j];
-    const long long cnt = (long long)*J.total;
-    qmerge_range(J.c.pix, (const double*)J.k.q64, cnt, J.c.n0, J.c.n1, J.q.q64, (b - cb[j]) * blockDim.x + threadIdx.x,
-                 J.cblocks * blockDim.x);
+    const QcutArgs a = J.k;
+    const QcutMerge M{J.c.pix, J.c.n0, J.c.n1, J.q.q64};
+    qcut_range<true>(a, M, (b - cb[j]) * blockDim.x + threadIdx.x, J.cblocks * blockDim.x);
 }
 
 // ---- host launchers ----
@@ -358,10 +394,14 @@ cudaError_t launch_cook(const CookArgs& a, int* tile_count, long long* tile_off,
     }
     if (ntiles > 0x7fffffffLL) return cudaErrorInvalidValue;
     k_flag_count<<<(unsigned)ntiles, 256, 0, st>>>(a.bflag, a.n, a.n0, a.n1, a.interior_only, tile_count);
-    k_tile_scan<<<1, 1024, 0, st>>>(tile_count, ntiles, tile_off, total);
     CookArgs b = a;
     b.tile_off = tile_off;
-    k_cook_write<<<(unsigned)ntiles, kTile, 0, st>>>(b);
+    if (ntiles <= kSelfScan) {
+        k_cook_write<true><<<(unsigned)ntiles, kTile, 0, st>>>(b, tile_count, total);
+    } else {
+        k_tile_scan<<<1, 1024, 0, st>>>(tile_count, ntiles, tile_off, total);
+        k_cook_write<false><<<(unsigned)ntiles, kTile, 0, st>>>(b, tile_count, total);
+    }
     return cudaGetLastError();
 }
 
@@ -369,8 +409,16 @@ long long cook_tiles(long long n) { return (n + kTile - 1) / kTile; }
 
 cudaError_t launch_qcut(const QcutArgs& a, bool f64, long long max_count, cudaStream_t st) {
     if (max_count <= 0) return cudaSuccess;
-    if (f64) k_qcut<true><<<grid_for(max_count, 256), 256, 0, st>>>(a);
-    else k_qcut<false><<<grid_for(max_count, 256), 256, 0, st>>>(a);
+    const QcutMerge none{nullptr, 0, 0, nullptr};
+    if (f64) k_qcut<true><<<grid_for(max_count, 256), 256, 0, st>>>(a, none);
+    else k_qcut<false><<<grid_for(max_count, 256), 256, 0, st>>>(a, none);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_qcut_merge(const QcutArgs& a, long long max_count, const long long* pix, int n0, int n1,
+                              double* qmap, cudaStream_t st) {
+    if (max_count <= 0) return cudaSuccess;
+    k_qcut<true><<<grid_for(max_count, 256), 256, 0, st>>>(a, QcutMerge{pix, n0, n1, qmap});
     return cudaGetLastError();
 }
 
@@ -397,8 +445,12 @@ cudaError_t launch_qpost_assemble(const QPostJob* jobs, const long long* begin, 
         if (grid[g] < 1 || grid[g] > 0x7fffffffLL) return cudaErrorInvalidValue;
     k_qcalc_jobs<<<(unsigned)grid[0], 256, 0, st>>>(jobs, begin, njobs);
     k_flag_count_jobs<<<(unsigned)grid[1], 256, 0, st>>>(jobs, begin, njobs);
-    k_tile_scan_jobs<<<(unsigned)njobs, 1024, 0, st>>>(jobs, begin, njobs);
-    k_cook_write_jobs<<<(unsigned)grid[1], kTile, 0, st>>>(jobs, begin, njobs);
+    if (grid[1] <= kSelfScan) {
+        k_cook_write_jobs<true><<<(unsigned)grid[1], kTile, 0, st>>>(jobs, begin, njobs);
+    } else {
+        k_tile_scan_jobs<<<(unsigned)njobs, 1024, 0, st>>>(jobs, begin, njobs);
+        k_cook_write_jobs<false><<<(unsigned)grid[1], kTile, 0, st>>>(jobs, begin, njobs);
+    }
     return cudaGetLastError();
 }
 
@@ -407,7 +459,6 @@ cudaError_t launch_qpost_pseudo(const QPostJob* jobs, const long long* begin, in
     if (njobs < 1) return cudaSuccess;
     if (grid[2] < 1 || grid[2] > 0x7fffffffLL) return cudaErrorInvalidValue;
     k_qcut_jobs<<<(unsigned)grid[2], 256, 0, st>>>(jobs, begin, njobs);
-    k_qmerge_jobs<<<(unsigned)grid[2], 256, 0, st>>>(jobs, begin, njobs);
     return cudaGetLastError();
 }
 

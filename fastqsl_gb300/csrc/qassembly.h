@@ -72,6 +72,9 @@ long long cook_tiles(long long n);
 cudaError_t launch_cook(const CookArgs& a, int* tile_count, long long* tile_off, unsigned long long* total,
                         cudaStream_t st);
 cudaError_t launch_qcut(const QcutArgs& a, bool f64, long long max_count, cudaStream_t st);
+// launch_qcut in FP64, each pixel's Q also written into the map (launch_qmerge_f64)
+cudaError_t launch_qcut_merge(const QcutArgs& a, long long max_count, const long long* pix, int n0, int n1,
+                              double* qmap, cudaStream_t st);
 cudaError_t launch_qmerge_f32(const long long* pix, const float* qcut, const unsigned long long* count_dev,
                               long long count, long long max_count, int n0, int n1, float* qfinal, cudaStream_t st);
 cudaError_t launch_qmerge_f64(const long long* pix, const double* qcut, const unsigned long long* count_dev,

@@ -525,6 +525,14 @@ int qsl_qcut(const float *start_x, const float *start_y, const float *start_z, c
              const float *Bz0_start, const float *Bz0_end, int64_t count, const unsigned long long *count_dev,
              int64_t max_count, double jac_scale, float *Qcut32, double *Qcut64, qsl_stream_t stream);
 
+/* qsl_qcut in FP64 and qsl_qmerge in one launch: each pixel's Q goes to
+ * Qcut64 and, at its `pix`, into Qfinal64 (nplanes, n0-2, n1-2). */
+int qsl_qcut_merge(const float *start_x, const float *start_y, const float *start_z, const int *flag_start,
+                   const float *end_x, const float *end_y, const float *end_z, const int *flag_end,
+                   const float *Bz0_start, const float *Bz0_end, int64_t count, const unsigned long long *count_dev,
+                   int64_t max_count, double jac_scale, const int64_t *pix, int n0, int n1, double *Qcut64,
+                   double *Qfinal64, qsl_stream_t stream);
+
 /* Replaces demo/Q_RKF45CuPy.ipynb cell 11: Qfinal (nplanes, n0-2, n1-2) gets
  * Qcut at every compacted interior pixel `pix`. */
 int qsl_qmerge(const int64_t *pix, const float *Qcut32, const double *Qcut64, int64_t count,
@@ -553,7 +561,7 @@ int qsl_plane_seeds(const double *center_h, const double *normal_h, const double
  * (qsl_plane_seeds) and tile order (qsl_tile_order), one batched main trace
  * (or windows of it), then per job Q (qsl_qcalc_plane, FP64) and the
  * pseudo-line compaction (qsl_cook_pseudo_line), one batched pseudo-line
- * trace, per job pseudo Q and merge (qsl_qcut, qsl_qmerge).  The Q maps
+ * trace, per job pseudo Q and merge (qsl_qcut_merge).  The Q maps
  * equal a batch of the same jobs built from those entries one by one, bit
  * for bit.  No device allocation, no synchronisation; a serving loop builds
  * a batch of small requests in a few launches per request.
