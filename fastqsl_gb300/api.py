@@ -660,9 +660,15 @@ class PlaneQBatch:
     def main_lines(self):
         return int(_lib.load().qsl_qmap_batch_lines(self.handle))
 
-    def run_main(self, stream=None, lo=0, hi=-1):
-        """The batched main trace, or the window [lo, hi) of its lines."""
-        _lib.check(_lib.load().qsl_qmap_batch_run_main(self.handle, int(lo), int(hi), self.max_blocks, self.occupancy,
+    def run_main(self, stream=None, lo=0, hi=-1, share=False):
+        """The batched main trace, or the window [lo, hi) of its lines.
+        share: other work is on the GPU; the launch then keeps to one thread
+        per line, where it would else give a line up to eight of the GPU's
+        idle lanes.  The results are the same."""
+        cap = self.max_blocks
+        if share:
+            cap = min(cap or 1 << 30, max(1, (self.main_lines + 127) // 128))
+        _lib.check(_lib.load().qsl_qmap_batch_run_main(self.handle, int(lo), int(hi), cap, self.occupancy,
                                                        stream_handle(stream)), "qsl_qmap_batch_run_main")
 
     def run_post(self, stream=None):

@@ -342,8 +342,12 @@ class QServer:
             fl.ready = torch.cuda.Event()
             fl.ready.record(st)
         else:
+            # alone, a batch may take every idle lane of the GPU; beside others
+            # that costs them more than it gives (10^4-3x10^4 seeds, p50 alone
+            # and at 1600 requests/s: 1.25 and 3.3 ms with all lanes always,
+            # 1.55 and 2.55 never, 1.25 and 2.55 ms so)
             with torch.cuda.stream(st):
-                qb.run_main(stream=st)
+                qb.run_main(stream=st, share=len(self.flights) > 1)
             self._post(fl)
 
     def idle(self):
