@@ -870,11 +870,11 @@ def main():
                                    "planes: issue active ~74 %, FMA pipe ~64 % of its cycles, L1 LSU wavefronts "
                                    "~76 % of peak)")
     # launches per step: main trace, qcalc, flag_count, tile_scan, cook_write,
-    # pseudo trace, qcut, qmerge (+ 2 memsets of the queue counters)
-    line["gpu_launches"] = 8 * args.steps
+    # pseudo trace, qcut with the merge (+ 2 memsets of the queue counters)
+    line["gpu_launches"] = 7 * args.steps
     line["config"]["autotune"] = res["autotune"]
     at = res["autotune"]
-    sched = "static lockstep" if at["schedule"] == "static" else f"work queue, {at['chunk']} lines per refill"
+    sched = "static lockstep" if at["schedule"] == "static" else f"work queue, {at['chunk']} lines per turn"
     line["config"]["schedule"] = (f"{sched}, {at['tile'][0]}x{at['tile'][1]} seed tiles in column order, "
                                   f"occupancy {at['occupancy']} ({'default' if args.no_autotune else 'autotuned'})")
     if acc:

@@ -601,7 +601,7 @@ class PlaneQBatch:
     seed grids, tile orders, job tables, batched traces and the batched Q
     assembly are laid out in one workspace allocation and queued by the C++
     library: two launches per job (seed grid, tile order), then the batch's
-    traces and six Q-assembly launches for all jobs, and no per-array host
+    traces and four or five Q-assembly launches for all jobs, and no per-array host
     bookkeeping.  The Q maps equal QBatch's on the same jobs bit for bit (the
     same trace kernels; the Q-assembly kernels' arithmetic per pixel).  Reference workflow per job: demo/Q_RKF45CuPy.ipynb
     cells 7-11.
@@ -671,10 +671,15 @@ class PlaneQBatch:
         _lib.check(_lib.load().qsl_qmap_batch_run_main(self.handle, int(lo), int(hi), cap, self.occupancy,
                                                        stream_handle(stream)), "qsl_qmap_batch_run_main")
 
-    def run_post(self, stream=None):
+    def run_post(self, stream=None, share=False):
         """Everything after the main trace: Q, pseudo-lines, merge; returns
-        the jobs' Q maps (views of the workspace)."""
-        _lib.check(_lib.load().qsl_qmap_batch_run_post(self.handle, self.max_blocks, self.occupancy,
+        the jobs' Q maps (views of the workspace).  share: as for run_main (a
+        launch held to fewer blocks than its lines fill gives a pseudo-line
+        one thread)."""
+        cap = self.max_blocks
+        if share:
+            cap = min(cap or 1 << 30, max(1, sum(4 * q.numel() for q in self.Q) // 256))
+        _lib.check(_lib.load().qsl_qmap_batch_run_post(self.handle, cap, self.occupancy,
                                                        stream_handle(stream)), "qsl_qmap_batch_run_post")
         return self.Q
 

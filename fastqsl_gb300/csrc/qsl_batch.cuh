@@ -24,7 +24,7 @@ struct BatchSlot {
 //
 // A job whose count comes from the device (n_dev) usually fills a small part
 // of its range, and the warps past it would start and exit.  When the whole
-// batch runs in one launch, its lines go to all the job's warps: directions
+// batch runs in one launch of its own, its lines go to all the job's warps: directions
 // to pairs of warps and up to four lanes per line, as in a launch of their
 // own (all after the main trace of two requests
 // of 17,000 seeds: 0.90 -> 0.75 ms).
@@ -81,9 +81,11 @@ __device__ __forceinline__ void batch_kernel_body(const TraceJob<F>* __restrict_
                                                   unsigned long long* samples, long long line_lo,
                                                   long long line_hi) {
     long long total = __ldg(begin + njobs);
-    const bool whole = line_lo == 0 && line_hi >= total;
-    total = line_hi < total ? line_hi : total;
     const long long warps = (long long)gridDim.x * (kTraceThreads / 32);
+    // fewer warps than lines fill: a cap on the grid, by a caller that shares
+    // the GPU with other launches
+    const bool whole = line_lo == 0 && line_hi >= total && 32 * warps >= total;
+    total = line_hi < total ? line_hi : total;
     const long long w = (long long)blockIdx.x * (kTraceThreads / 32) + (threadIdx.x >> 5);
     // lanes to spare: the directions over warp pairs, fewer lines per warp
     const bool split = splits(total - line_lo, warps);

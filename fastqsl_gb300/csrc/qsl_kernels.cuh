@@ -97,8 +97,8 @@ static cudaError_t launch_scott(const ScottJob<F>& J, int grad, bool twist, long
     return cudaGetLastError();
 }
 
-// Batched trace: one line per thread; MINB resident blocks per SM the
-// register allocation must allow (6-10; the autotuner picks, 8 by default).
+// Batched trace; MINB resident blocks per SM the
+// register allocation must allow (6-10; the autotuner picks, 6 by default).
 template <bool TWIST, class F, int MINB>
 __global__ void __launch_bounds__(kTraceBlock, MINB) k_trace_batch(const TraceJob<F>* __restrict__ jobs,
                                                                     const long long* __restrict__ begin, int njobs,
