@@ -182,9 +182,10 @@ class QServer:
         self._next_stream = [0] * len(self.classes)
         self.s_len, self.h_min, self.h_max = s_len, h_min, h_max
         self.tile = tile
-        # batches of all but the smallest class keep at most this many of
-        # the 8 resident block slots per SM, so the smallest requests' blocks
-        # (on the highest-priority stream) start at once (0 = no cap)
+        # batches of all but the smallest class, where they run whole, keep at
+        # most this many blocks per SM (6 are resident at the batched kernels'
+        # default budget), each looping over its lines; fewer leave slots in
+        # which the smallest requests' blocks start at once (0 = no cap)
         self.big_blocks_per_sm = int(big_blocks_per_sm)
         # main traces of classes > 0 run as windows of chunk_lines lines (a
         # multiple of 32; 0 = one launch per batch)
