@@ -48,15 +48,16 @@ __device__ __forceinline__ BatchSlot batch_slot(const TraceJob<F>& J, long long 
 }
 
 template <bool TWIST, class F>
-__device__ __forceinline__ void batch_line(const TraceJob<F>& J, const BatchSlot& slot, long long n, long long left,
-                                           unsigned& ns) {
+__device__ __forceinline__ void batch_line(const TraceJob<F>& J, const BatchSlot& slot, long long n, long long skip,
+                                           long long left, unsigned& ns) {
     F f = J.f;
     if (f.d.nx < 2 || f.d.ny < 2 || f.d.nz < 2) return;
     const int lane = threadIdx.x & 31;
     const long long line = slot.first + lane / slot.spread;
     if (slot.first >= n) return;  // past the job's lines (a whole warp, or a whole pair)
-    // else lanes past the job's lines or the window, or between spread lines
-    const bool valid = lane % slot.spread == 0 && line < n && lane / slot.spread < left;
+    // else lanes past the job's lines, outside the window, or between spread lines
+    const int k = lane / slot.spread;
+    const bool valid = lane % slot.spread == 0 && line < n && k >= skip && k < left;
     const long long i = (valid && J.order) ? (long long)__ldg(J.order + line) : line;
     const bool tw_on = TWIST && J.s.twist_on != 0;
     store_prepare(f);
@@ -73,8 +74,9 @@ __device__ __forceinline__ void batch_line(const TraceJob<F>& J, const BatchSlot
 
 // begin[j]: first line of job j (multiples of 32, increasing); begin[njobs]:
 // the total.  Each job's TraceJob sits in device memory.  Only the lines of
-// the window [line_lo, line_hi) run (a multiple of 32 for line_lo keeps every
-// warp inside one job).
+// the window [line_lo, line_hi) run.  The warps' lines are counted from the
+// multiple of 32 at or below line_lo, whatever the window, so that every warp
+// stays inside one job; lanes below line_lo have no line.
 template <bool TWIST, class F>
 __device__ __forceinline__ void batch_kernel_body(const TraceJob<F>* __restrict__ jobs,
                                                   const long long* __restrict__ begin, int njobs,
@@ -88,13 +90,14 @@ __device__ __forceinline__ void batch_kernel_body(const TraceJob<F>* __restrict_
     total = line_hi < total ? line_hi : total;
     const long long w = (long long)blockIdx.x * (kTraceThreads / 32) + (threadIdx.x >> 5);
     // lanes to spare: the directions over warp pairs, fewer lines per warp
-    const bool split = splits(total - line_lo, warps);
-    const int spread = split ? spread_of(total - line_lo, warps) : 1;
+    const long long base = line_lo & ~31LL;
+    const bool split = splits(total - base, warps);
+    const int spread = split ? spread_of(total - base, warps) : 1;
     const int lines = 32 / spread;
     const long long stride = warps * lines / (split ? 2 : 1);
     unsigned ns = 0;
     unsigned long long ns_total = 0;
-    for (long long g = line_lo + (split ? w >> 1 : w) * lines; g < total; g += stride) {
+    for (long long g = base + (split ? w >> 1 : w) * lines; g < total; g += stride) {
         int lo = 0, hi = njobs - 1;  // last j with begin[j] <= g
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -110,7 +113,7 @@ __device__ __forceinline__ void batch_kernel_body(const TraceJob<F>* __restrict_
         }
         const BatchSlot slot =
             split ? BatchSlot{g - b, true, spread} : batch_slot(J, n, g, b, __ldg(begin + lo + 1) - b, whole);
-        batch_line<TWIST>(J, slot, n, split | !slot.split ? total - g : 32, ns);
+        batch_line<TWIST>(J, slot, n, line_lo - g, split | !slot.split ? total - g : 32, ns);
         ns_total += ns;
         ns = 0;
     }

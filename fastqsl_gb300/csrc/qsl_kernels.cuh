@@ -139,7 +139,7 @@ static cudaError_t launch_batch(const TraceJob<F>* jobs, const long long* begin,
     if (line_lo >= line_hi) return cudaSuccess;
     const int resident = persistent_grid(batch_kernel<F>(occupancy, twist), kTraceBlock);
     if (resident <= 0) return cudaErrorInvalidConfiguration;
-    int grid = static_grid(line_hi - line_lo, resident);
+    int grid = static_grid(line_hi - (line_lo & ~31LL), resident);  // (batch_kernel_body's first line)
     if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;  // the grid-stride loop covers the rest
     switch (occupancy) {
         case 7: launch_batch_minb<F, 7>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;

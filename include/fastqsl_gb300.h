@@ -279,8 +279,8 @@ typedef struct qsl_batch_info {
 int qsl_batch_pack(const qsl_batch_job *jobs_h, int njobs, void *table_h, int64_t table_bytes,
                    qsl_batch_info *info_h);
 /* qsl_batch_run over the lines [line_lo, line_hi) of each store type's line
- * space (line_hi < 0: to the end; line_lo a multiple of 32 keeps each warp
- * inside one job) with at most max_blocks resident 128-thread blocks per
+ * space (any line_lo, a multiple of 32 wastes no lanes; line_hi < 0: to the
+ * end) with at most max_blocks resident 128-thread blocks per
  * launch (0 = no limit; the blocks then loop over the lines).  A serving loop
  * runs a large batch as a sequence of such windows, so that small requests
  * never share the GPU with more than a window of it, and caps its resident
