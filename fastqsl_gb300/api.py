@@ -660,26 +660,24 @@ class PlaneQBatch:
     def main_lines(self):
         return int(_lib.load().qsl_qmap_batch_lines(self.handle))
 
+    def _limit(self, share):
+        """The block limit of a launch: any limit keeps it to one thread per
+        line (qsl_batch_run_window), one that no grid reaches does only that."""
+        return self.max_blocks or (1 << 30 if share else 0)
+
     def run_main(self, stream=None, lo=0, hi=-1, share=False):
         """The batched main trace, or the window [lo, hi) of its lines.
         share: other work is on the GPU; the launch then keeps to one thread
         per line, where it would else give a line up to eight of the GPU's
         idle lanes.  The results are the same."""
-        cap = self.max_blocks
-        if share:
-            cap = min(cap or 1 << 30, max(1, (self.main_lines + 127) // 128))
-        _lib.check(_lib.load().qsl_qmap_batch_run_main(self.handle, int(lo), int(hi), cap, self.occupancy,
-                                                       stream_handle(stream)), "qsl_qmap_batch_run_main")
+        _lib.check(_lib.load().qsl_qmap_batch_run_main(self.handle, int(lo), int(hi), self._limit(share),
+                                                       self.occupancy, stream_handle(stream)),
+                   "qsl_qmap_batch_run_main")
 
     def run_post(self, stream=None, share=False):
         """Everything after the main trace: Q, pseudo-lines, merge; returns
-        the jobs' Q maps (views of the workspace).  share: as for run_main (a
-        launch held to fewer blocks than its lines fill gives a pseudo-line
-        one thread)."""
-        cap = self.max_blocks
-        if share:
-            cap = min(cap or 1 << 30, max(1, sum(4 * q.numel() for q in self.Q) // 256))
-        _lib.check(_lib.load().qsl_qmap_batch_run_post(self.handle, cap, self.occupancy,
+        the jobs' Q maps (views of the workspace).  share: as for run_main."""
+        _lib.check(_lib.load().qsl_qmap_batch_run_post(self.handle, self._limit(share), self.occupancy,
                                                        stream_handle(stream)), "qsl_qmap_batch_run_post")
         return self.Q
 
@@ -833,8 +831,8 @@ class BatchPlan:
 
     def launch(self, samples=None, stream=None, max_blocks=0, lo=0, hi=-1, occupancy=0):
         """Lines [lo, hi) of the batch (hi < 0: all); max_blocks > 0: at most
-        that many resident blocks (they loop over the lines), leaving the rest
-        of the GPU's block slots free; occupancy: the kernels' register budget
+        that many resident blocks (they loop over the lines, one thread per
+        line), leaving the rest of the GPU's block slots free; occupancy: the kernels' register budget
         in resident blocks per SM (6-10, 0 = 6)."""
         _lib.check(_lib.load().qsl_batch_run_window(self._dev.data_ptr(), ctypes.byref(self.info), ptr(samples),
                                                     int(lo), int(hi), int(max_blocks), int(occupancy),

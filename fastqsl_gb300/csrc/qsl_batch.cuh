@@ -72,27 +72,35 @@ __device__ __forceinline__ void batch_line(const TraceJob<F>& J, const BatchSlot
         [&J]() { return J.s.tol_coef; }, [&J]() { return v3(J.s.cross[0], J.s.cross[1], J.s.cross[2]); }, tw_on, ns);
 }
 
+// The shape of a launch of n lines of the batch: without spare lanes one
+// thread per line, whatever the grid.
+__host__ __device__ __forceinline__ LaunchShape batch_shape(long long n, long long warps, bool lanes_free) {
+    return lanes_free ? launch_shape(n, warps) : LaunchShape{false, 1};
+}
+
 // begin[j]: first line of job j (multiples of 32, increasing); begin[njobs]:
 // the total.  Each job's TraceJob sits in device memory.  Only the lines of
 // the window [line_lo, line_hi) run.  The warps' lines are counted from the
 // multiple of 32 at or below line_lo, whatever the window, so that every warp
-// stays inside one job; lanes below line_lo have no line.
+// stays inside one job; lanes below line_lo have no line.  lanes_free: the
+// launch may give a line several lanes (a caller that limits its blocks shares
+// the GPU with other launches: then it may not).
 template <bool TWIST, class F>
 __device__ __forceinline__ void batch_kernel_body(const TraceJob<F>* __restrict__ jobs,
                                                   const long long* __restrict__ begin, int njobs,
                                                   unsigned long long* samples, long long line_lo,
-                                                  long long line_hi) {
+                                                  long long line_hi, bool lanes_free) {
     long long total = __ldg(begin + njobs);
     const long long warps = (long long)gridDim.x * (kTraceThreads / 32);
-    // fewer warps than lines fill: a cap on the grid, by a caller that shares
-    // the GPU with other launches
-    const bool whole = line_lo == 0 && line_hi >= total && 32 * warps >= total;
+    // the whole batch in this launch, with the GPU's idle lanes at its disposal
+    const bool whole = lanes_free && line_lo == 0 && line_hi >= total && 32 * warps >= total;
     total = line_hi < total ? line_hi : total;
     const long long w = (long long)blockIdx.x * (kTraceThreads / 32) + (threadIdx.x >> 5);
     // lanes to spare: the directions over warp pairs, fewer lines per warp
     const long long base = line_lo & ~31LL;
-    const bool split = splits(total - base, warps);
-    const int spread = split ? spread_of(total - base, warps) : 1;
+    const LaunchShape shape = batch_shape(total - base, warps, lanes_free);
+    const bool split = shape.split;
+    const int spread = shape.spread;
     const int lines = 32 / spread;
     const long long stride = warps * lines / (split ? 2 : 1);
     unsigned ns = 0;

@@ -35,6 +35,15 @@ inline int static_grid(long long n, int resident) {
     return (int)(g < 1 ? 1 : (g > (1 << 30) ? (1 << 30) : g));
 }
 
+// Grid of a batched launch of n lines.  A limit on its blocks (max_blocks > 0)
+// comes from a caller with other work on the GPU: one thread per line then,
+// on at most that many blocks, which loop over the lines.
+inline int batch_grid(long long n, int resident, int max_blocks) {
+    if (max_blocks <= 0) return static_grid(n, resident);
+    const long long g = (n + kTraceBlock - 1) / kTraceBlock;
+    return (int)(g < 1 ? 1 : (g > max_blocks ? max_blocks : (g > (1 << 30) ? (1 << 30) : g)));
+}
+
 // trace_exact.cu (compiled with -fmad=false)
 cudaError_t launch_trace_exact(const TraceJob<FieldSoA>& J, bool twist, Schedule sched, long long n_host,
                                cudaStream_t st);

@@ -97,21 +97,22 @@ static cudaError_t launch_scott(const ScottJob<F>& J, int grad, bool twist, long
     return cudaGetLastError();
 }
 
-// Batched trace; MINB resident blocks per SM the
-// register allocation must allow (6-10; the autotuner picks, 6 by default).
+// Batched trace; MINB resident blocks per SM the register allocation must
+// allow (6-10; the autotuner picks, 6 by default).
 template <bool TWIST, class F, int MINB>
 __global__ void __launch_bounds__(kTraceBlock, MINB) k_trace_batch(const TraceJob<F>* __restrict__ jobs,
                                                                     const long long* __restrict__ begin, int njobs,
                                                                     unsigned long long* samples, long long line_lo,
-                                                                    long long line_hi) {
-    batch_kernel_body<TWIST>(jobs, begin, njobs, samples, line_lo, line_hi);
+                                                                    long long line_hi, bool lanes_free) {
+    batch_kernel_body<TWIST>(jobs, begin, njobs, samples, line_lo, line_hi, lanes_free);
 }
 
 template <class F, int MINB>
 static void launch_batch_minb(int grid, const TraceJob<F>* jobs, const long long* begin, int njobs, bool twist,
-                              unsigned long long* samples, long long line_lo, long long line_hi, cudaStream_t st) {
-    if (twist) k_trace_batch<true, F, MINB><<<grid, kTraceBlock, 0, st>>>(jobs, begin, njobs, samples, line_lo, line_hi);
-    else k_trace_batch<false, F, MINB><<<grid, kTraceBlock, 0, st>>>(jobs, begin, njobs, samples, line_lo, line_hi);
+                              unsigned long long* samples, long long line_lo, long long line_hi, bool lanes_free,
+                              cudaStream_t st) {
+    auto k = twist ? k_trace_batch<true, F, MINB> : k_trace_batch<false, F, MINB>;
+    k<<<grid, kTraceBlock, 0, st>>>(jobs, begin, njobs, samples, line_lo, line_hi, lanes_free);
 }
 
 template <class F, int MINB>
@@ -139,14 +140,14 @@ static cudaError_t launch_batch(const TraceJob<F>* jobs, const long long* begin,
     if (line_lo >= line_hi) return cudaSuccess;
     const int resident = persistent_grid(batch_kernel<F>(occupancy, twist), kTraceBlock);
     if (resident <= 0) return cudaErrorInvalidConfiguration;
-    int grid = static_grid(line_hi - (line_lo & ~31LL), resident);  // (batch_kernel_body's first line)
-    if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;  // the grid-stride loop covers the rest
+    const int grid = batch_grid(line_hi - (line_lo & ~31LL), resident, max_blocks);  // (batch_kernel_body's first line)
+    const bool free = max_blocks <= 0;
     switch (occupancy) {
-        case 7: launch_batch_minb<F, 7>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
-        case 9: launch_batch_minb<F, 9>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
-        case 10: launch_batch_minb<F, 10>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
-        case 8: launch_batch_minb<F, 8>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
-        default: launch_batch_minb<F, 6>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, st); break;
+        case 7: launch_batch_minb<F, 7>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, free, st); break;
+        case 8: launch_batch_minb<F, 8>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, free, st); break;
+        case 9: launch_batch_minb<F, 9>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, free, st); break;
+        case 10: launch_batch_minb<F, 10>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, free, st); break;
+        default: launch_batch_minb<F, 6>(grid, jobs, begin, njobs, twist, samples, line_lo, line_hi, free, st); break;
     }
     return cudaGetLastError();
 }

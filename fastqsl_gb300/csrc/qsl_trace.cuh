@@ -1128,6 +1128,16 @@ __host__ __device__ __forceinline__ int spread_of(long long n, long long warps) 
     return s;
 }
 
+// How a launch of n lines on `warps` warps shares its lanes out.
+struct LaunchShape {
+    bool split;
+    int spread;
+};
+__host__ __device__ __forceinline__ LaunchShape launch_shape(long long n, long long warps) {
+    const bool split = splits(n, warps);
+    return {split, split ? spread_of(n, warps) : 1};
+}
+
 // The tracer kernel: every warp takes 32 lines at a time and traces them in
 // lockstep.  QUEUE = true: persistent grid; a warp takes chunks of J.chunk
 // consecutive lines from the device counter J.queue, so uneven lines even
@@ -1183,8 +1193,9 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
     unsigned ns = 0;
     const int lane_id = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (blockDim.x / 32);
-    const bool split = splits(n_of(), warps);
-    const int spread = split ? spread_of(n_of(), warps) : 1;
+    const LaunchShape shape = launch_shape(n_of(), warps);
+    const bool split = shape.split;
+    const int spread = shape.spread;
     const int lines = 32 / spread;  // of a warp
     const bool queued = QUEUE && !split;
     // the warp's first line, and the end of its chunk

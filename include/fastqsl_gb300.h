@@ -285,10 +285,10 @@ int qsl_batch_pack(const qsl_batch_job *jobs_h, int njobs, void *table_h, int64_
  * runs a large batch as a sequence of such windows, so that small requests
  * never share the GPU with more than a window of it, and caps its resident
  * blocks below the GPU's capacity.  Without a limit a launch whose lines do
- * not fill the GPU gives each of them up to eight lanes; a limit of one block
- * per 128 lines keeps it to one thread per line, for callers with other work
- * on the GPU (the results are the same).  occupancy: the register budget of
- * the batched kernels, for this many resident 128-thread blocks per SM (6-10;
+ * not fill the GPU gives each of them up to eight lanes; with one, however
+ * large, it keeps to one thread per line, for callers with other work on the
+ * GPU (the results are the same).  occupancy: the register budget of the
+ * batched kernels, for this many resident 128-thread blocks per SM (6-10;
  * 0 = 6). */
 int qsl_batch_run_window(const void *table_dev, const qsl_batch_info *info_h, unsigned long long *samples_dev,
                          int64_t line_lo, int64_t line_hi, int max_blocks, int occupancy, qsl_stream_t stream);
@@ -601,9 +601,8 @@ int qsl_qmap_batch_run_main(const qsl_qmap_batch_t *batch, int64_t line_lo, int6
                             int occupancy, qsl_stream_t stream);
 /* Everything after the main trace: Q, pseudo-lines and merge of every job
  * (the Q assembly, compaction, pseudo Q with the merge as one launch each
- * for the whole batch, the pseudo-line trace as one batched trace; with a
- * limit below one block per 128 lines of its capacity a pseudo-line keeps to
- * one thread). */
+ * for the whole batch, the pseudo-line trace as one batched trace),
+ * max_blocks / occupancy as in qsl_batch_run_window. */
 int qsl_qmap_batch_run_post(const qsl_qmap_batch_t *batch, int max_blocks, int occupancy, qsl_stream_t stream);
 /* Device address of job k's Q, float64 (nplanes, n0 - 2, n1 - 2) inside the workspace. */
 double *qsl_qmap_batch_q(const qsl_qmap_batch_t *batch, int job);
