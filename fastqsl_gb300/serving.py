@@ -269,7 +269,8 @@ class QServer:
                 ws = wss[k]
                 ws.wait_event(fl.ready)
                 with torch.cuda.stream(ws):
-                    fl.qb.run_main(stream=ws, lo=fl.next_lo, hi=hi)
+                    # (a batch's last window may leave lanes free)
+                    fl.qb.run_main(stream=ws, lo=fl.next_lo, hi=hi, share=len(self.flights) > 1)
                     ev = torch.cuda.Event()
                     ev.record(ws)
                 fl.windows.append(ev)
