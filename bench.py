@@ -874,7 +874,7 @@ def main():
     line["gpu_launches"] = 7 * args.steps
     line["config"]["autotune"] = res["autotune"]
     at = res["autotune"]
-    sched = "static lockstep" if at["schedule"] == "static" else f"work queue, {at['chunk']} lines per turn"
+    sched = "static lockstep" if at["schedule"] == "static" else f"work queue, at most {at['chunk']} lines at a time"
     line["config"]["schedule"] = (f"{sched}, {at['tile'][0]}x{at['tile'][1]} seed tiles in column order, "
                                   f"occupancy {at['occupancy']} ({'default' if args.no_autotune else 'autotuned'})")
     if acc:

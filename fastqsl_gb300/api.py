@@ -248,8 +248,8 @@ def trace(field: FieldStore, xs, ys, zs, params: TraceParams | None = None, s_le
     device counter holding the seed count (outputs must then hold the largest
     count).  `samples`: optional int64 CUDA tensor accumulating the number of
     trilinear samples taken.  `order`: optional int32 permutation; line k
-    traces seed order[k] (see tile_order).  `chunk`: lines a warp takes from
-    the queue at a time (0: 32).
+    traces seed order[k] (see tile_order).  `chunk`: the most lines a warp
+    takes from the queue at a time (0, and above 32: 32).
     `curB`: the current density for the twist integral, as three x-fastest
     float32 device arrays or as a FieldStore of the field's layout and shape
     (qsl_trace_cur: each current sample costs a field sample).  `status`:

@@ -9,8 +9,7 @@ spread evenly over the stack) for each candidate
 * resident-block budget — registers per thread sized for 0 (compiler's
   choice), 6, 7, 8, 9 or 10 blocks of 128 threads per SM,
 * schedule — static lockstep (one line per thread) against the device work
-  queue with 32, 128 or 512 lines per turn of a warp (32 of them at a time,
-  in lockstep), on the best tile and budget,
+  queue, on the best tile and budget,
 
 and keeps the fastest.  Results are cached per (device, store layout, field
 shape, integrator, plane shape).  tune_batch does the same for the batched
@@ -29,7 +28,7 @@ from . import api
 
 TILES = ((8, 8), (4, 8), (16, 16))
 OCCUPANCIES = (0, 6, 7, 8, 9, 10)
-QUEUE_CHUNKS = (32, 128, 512)
+QUEUE_CHUNKS = (32,)  # (a warp takes no more than 32 lines at a time)
 BATCH_OCCUPANCIES = (6, 7, 8, 9, 10)
 
 _cache: dict = {}
@@ -43,7 +42,7 @@ def _key(field, params, n0, n1):
 def tune_trace(field, xs, ys, zs, params, n0, n1, nplanes, s_len=0.25, tol_coef=1.0, cross_dir=(0.0, 0.0, 1.0),
                sample_planes=4, reps=2, tiles=TILES, occupancies=OCCUPANCIES, chunks=QUEUE_CHUNKS, use_cache=True):
     """Returns {'tile': (ty, tx), 'occupancy': k, 'schedule': 'static' or
-    'queue', 'chunk': lines per turn, 'ms': t, 'table': {...}} for the
+    'queue', 'chunk': most lines a warp takes at a time, 'ms': t, 'table': {...}} for the
     fastest candidate on `sample_planes` planes evenly spaced over the stack
     (lines from the bottom and the middle of a cube differ in length and
     spread)."""

@@ -9,9 +9,10 @@
 // backward; the footpoints, the samples of B and the outputs follow once for
 // the whole warp (trace_lines).  Where the launch has two threads per line,
 // the directions go to a pair of warps instead.  Static: the warp's lines
-// follow from its index; queue: a persistent grid whose warps take chunks of
-// lines from a device counter, for device-side counts and for lines whose
-// lengths differ by orders of magnitude between warps.
+// follow from its index; queue: a persistent grid whose warps take lines from
+// a device counter, new ones for the lanes that wait when the rest of a warp
+// takes too long (trace_queue), for device-side counts and for lines whose
+// lengths differ by orders of magnitude.
 //
 // What it replaced: every lane taking its next line from the queue as its
 // own ended, and doing its line's end then and there.  A warp's lanes were
@@ -94,7 +95,7 @@ struct TraceJob {
     unsigned long long* queue;    // work counter, zero at launch; null = static
     unsigned long long* samples;  // optional: total field samples
     const unsigned* order;        // optional: line k traces seed order[k] and writes its outputs there
-    int chunk;                    // lines a warp takes from the queue at a time (QUEUE; 0 = 32)
+    int chunk;                    // most lines a warp takes from the queue at a time (QUEUE; 0 = 32)
     int occupancy;                // resident-block variant of the fast kernels (0 = default)
 };
 
@@ -984,6 +985,7 @@ struct Stash {
     float lc;
     typename Lane<EXACT>::len_t len;
     double tw;
+    long long line;  // trace_queue: the lane's line (of S[0])
 };
 template <bool EXACT, bool TWIST>
 __device__ __forceinline__ void stash_put(Stash<EXACT>& S, const Lane<EXACT>& L) {
@@ -1112,6 +1114,97 @@ __device__ __forceinline__ void trace_lines(const F& f, const TraceJob<F>& J, lo
     ns += lines_finish<EXACT, TWIST>(f, J, S, i, valid, split, nrm_of(), tw_on);
 }
 
+__device__ __forceinline__ unsigned lanemask_lt() {
+    unsigned m;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    return m;
+}
+
+// The work-queue schedule, for more lines than the grid has lanes: a warp
+// takes lines from the device counter for all its lanes, traces them in
+// lockstep, and takes new ones for the lanes whose lines have ended once too
+// many wait.  The ended lines' footpoints, samples of B and outputs are done
+// then, for all of them at once.
+//
+// When it refills: a partial refill costs the coherence of a warp of
+// neighbours and does the ends for a part of its lanes, so it has to be
+// worth that.  kRefillLanes idle lanes; kRefillIdle looks, kRefillSteps trial
+// steps apart, summed over the idle lanes (64 steps of the whole warp); and
+// idle lane steps of a 1 / (1 + kRefillShare) part of all since the last
+// refill.  200,000 lines, ms, one refill per line as it ends / none before the
+// last line of 32 / this: a field whose lines are 3 % ropes of ten times the
+// mean length, bricks 8.0 / 9.8 / 6.7, float4 7.6 / 11.2 / 7.3, drop-in RKF45
+// 480 / 146 / 130; seeds anywhere in a charge field's volume 3.6 / 3.5 / 3.4,
+// 4.9 / 5.1 / 4.7, 37 / 11.5 / 9.3; its bottom plane in random order 1.9 /
+// 2.2 / 1.65, row by row 1.7 / 1.43 / 1.45.  What it costs: planes that are
+// coherent and even, 258 x 258 x 32 seeds on bricks in tile order 13.4 -> 14.0
+// (none -> this; 12.4 static), drop-in twist on 201 x 203 x 4 seeds 2.59 ->
+// 2.62.  Without the second and third rule (16 idle lanes alone) those two
+// were 14.6 and 2.67.
+constexpr int kRefillSteps = 8;
+constexpr int kRefillLanes = 16;
+constexpr unsigned kRefillIdle = 256;
+constexpr unsigned kRefillShare = 2;
+template <bool EXACT, bool TWIST, class F, class N, class SL, class TC, class NR>
+__device__ __forceinline__ void trace_queue(const F& f, const TraceJob<F>& J, const N& n_of,
+                                            const LenLimit<EXACT>& limit, const SL& s_len_of, const TC& tol_coef_of,
+                                            const NR& nrm_of, bool tw_on, unsigned& ns) {
+    Lane<EXACT> L;
+    Stash<EXACT> S[2];
+    bool active = false, ended = false;
+    bool drained = false;  // (warp-uniform) the counter is past the last line
+    while (true) {
+        if (__any_sync(0xffffffffu, ended)) {
+            ns += lines_finish<EXACT, TWIST>(f, J, S, S[0].line, ended, false, nrm_of(), tw_on);
+            ended = false;
+            // a lane's sample count nears 32 bits: hand it over (exact while
+            // one line takes fewer than 5e8 trial steps)
+            if (ns > (1u << 30)) {
+                if (J.samples) atomicAdd(J.samples, (unsigned long long)ns);
+                ns = 0;
+            }
+        }
+        unsigned want = __ballot_sync(0xffffffffu, !active);
+        while (want != 0u && !drained) {
+            // no more than the idle lanes: what a warp held back for later
+            // (a chunk of 256) waited while others had nothing left
+            int take = __popc(want);
+            if (J.chunk > 0 && take > J.chunk) take = J.chunk;
+            unsigned long long base = 0;
+            if ((threadIdx.x & 31) == 0) base = atomicAdd(J.queue, (unsigned long long)take);
+            const long long first = (long long)__shfl_sync(0xffffffffu, base, 0), n = n_of();
+            drained = first + take >= n;
+            const int rank = __popc(want & lanemask_lt());
+            if (!active && rank < take && first + rank < n) {
+                const long long i = J.order ? (long long)__ldg(J.order + first + rank) : first + rank;
+                S[0].line = i;
+                lane_begin<EXACT>(f, J, L, i, 1, s_len_of(), tol_coef_of(), nrm_of(), ns);
+                active = true;
+            }
+            want = __ballot_sync(0xffffffffu, !active);
+        }
+        if (!__any_sync(0xffffffffu, active)) break;
+        int idle;
+        unsigned busy_steps = 0, idle_steps = 0;
+        do {
+            for (int k = drained ? 0x7fffffff : kRefillSteps; active && k > 0; --k) {
+                if (!lane_step<EXACT, TWIST>(f, J, L, limit, tw_on, ns)) continue;
+                stash_put<EXACT, TWIST>(S[L.dsign >> 31], L);
+                if (L.dsign == 0) {
+                    lane_turn(J, L, S[0].line, s_len_of(), ns);
+                } else {
+                    active = false;
+                    ended = true;
+                }
+            }
+            idle = __popc(__ballot_sync(0xffffffffu, !active));
+            idle_steps += idle;
+            busy_steps += 32 - idle;
+        } while (idle < 32 && (drained || idle < kRefillLanes || idle_steps < kRefillIdle ||
+                               kRefillShare * idle_steps < busy_steps));
+    }
+}
+
 // Lanes a line takes in a launch of n lines (or capacity for as many) on
 // `warps` warps, the first of them active: the launch splits the directions
 // over warp pairs where it has two lanes per line, and gives every line two
@@ -1138,14 +1231,15 @@ __host__ __device__ __forceinline__ LaunchShape launch_shape(long long n, long l
     return {split, split ? spread_of(n, warps) : 1};
 }
 
-// The tracer kernel: every warp takes 32 lines at a time and traces them in
-// lockstep.  QUEUE = true: persistent grid; a warp takes chunks of J.chunk
-// consecutive lines from the device counter J.queue, so uneven lines even
-// out over the warps.  QUEUE = false: line = global thread index + k * total
-// threads.  A launch whose grid has two threads per line splits the
-// directions over warp pairs (trace_lines).  Lines are visited in J.order
-// when it is set.  TWIST compiles the twist integral in; it runs when the
-// runtime flag is set.
+// The tracer kernel.  QUEUE = true and more lines than the grid has lanes:
+// warps take lines from the device counter J.queue (trace_queue).  Else every
+// warp takes 32 lines at a time and traces them in lockstep, line = global
+// thread index + k * total threads; a launch whose grid has two threads per
+// line splits the directions over warp pairs (trace_lines).  (A queue launch
+// with a lane for every line: a plane of 250 x 300 seeds on a stretched grid
+// 1.24 ms from the counter, 1.19 so.)  Lines are visited in J.order when it
+// is set.  TWIST compiles the twist integral in; it runs when the runtime
+// flag is set.
 template <bool EXACT, bool TWIST, bool QUEUE, class F>
 __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
     F f = J.f;
@@ -1197,33 +1291,20 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
     const bool split = shape.split;
     const int spread = shape.spread;
     const int lines = 32 / spread;  // of a warp
-    const bool queued = QUEUE && !split;
-    // the warp's first line, and the end of its chunk
-    long long line = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), end = 0;
-    line = queued ? 0 : (split ? line >> 1 : line) * lines;
-    while (true) {
-        if (queued && line >= end) {
-            // lines per turn of the queue: the caller's choice, else the
-            // warp's 32 (256 left the 128 x 128 plane on 64 of 2432 warps, 64
-            // a map of 131,072 seeds on 2048)
-            const long long chunk = J.chunk > 0 ? J.chunk : 32;
-            unsigned long long base = 0;
-            if (lane_id == 0) base = atomicAdd(J.queue, (unsigned long long)chunk);
-            line = (long long)__shfl_sync(0xffffffffu, base, 0);
-            end = min(line + chunk, n_of());
+    if (QUEUE && n_of() > 32 * warps) {
+        trace_queue<EXACT, TWIST>(f, J, n_of, limit, s_len_of, tol_coef_of, nrm_of, tw_on, ns);
+    } else {
+        long long line = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+        for (line = (split ? line >> 1 : line) * lines; line < n_of(); line += warps * lines / (split ? 2 : 1)) {
+            const long long slot = line + lane_id / spread;
+            const bool valid = lane_id % spread == 0 && slot < n_of();
+            const long long i = (valid && J.order) ? (long long)__ldg(J.order + slot) : slot;
+            trace_lines<EXACT, TWIST>(f, J, i, valid, split, limit, s_len_of, tol_coef_of, nrm_of, tw_on, ns);
+            if (ns > (1u << 30)) {  // (as in trace_queue)
+                if (J.samples) atomicAdd(J.samples, (unsigned long long)ns);
+                ns = 0;
+            }
         }
-        if (line >= n_of()) break;
-        const long long slot = line + lane_id / spread;
-        const bool valid = lane_id % spread == 0 && slot < (queued ? end : n_of());
-        const long long i = (valid && J.order) ? (long long)__ldg(J.order + slot) : slot;
-        trace_lines<EXACT, TWIST>(f, J, i, valid, split, limit, s_len_of, tol_coef_of, nrm_of, tw_on, ns);
-        // a lane's sample count nears 32 bits: hand it over (exact while one
-        // line takes fewer than 5e8 trial steps)
-        if (ns > (1u << 30)) {
-            if (J.samples) atomicAdd(J.samples, (unsigned long long)ns);
-            ns = 0;
-        }
-        line += queued ? 32 : warps * lines / (split ? 2 : 1);
     }
     if (J.samples) {
         // one atomic per warp (blocks are whole warps; every lane gets here)

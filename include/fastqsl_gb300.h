@@ -211,7 +211,7 @@ typedef struct qsl_trace_io {
 /* Scheduling of a trace launch (host struct; pointers are device pointers). */
 typedef struct qsl_sched {
     int32_t schedule;            /* qsl_schedule */
-    int32_t chunk;               /* QUEUE: lines a warp takes at a time (0 = 32) */
+    int32_t chunk;               /* QUEUE: most lines a warp takes at a time (0, > 32 = 32) */
     const uint32_t *order;       /* optional: line k traces seed order[k] and writes its outputs at
                                     order[k] (a permutation of [0, n)); visiting seeds in compact
                                     tiles keeps a warp's gathers coherent */
