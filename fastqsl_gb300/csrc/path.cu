@@ -96,11 +96,14 @@ __device__ __forceinline__ bool in_range(const PathRun& R, long long idx) {
 // RK4_bline (MagTool.py:24-34), one thread per seed and run.  A warp's FP64
 // operations take this GPU's FP64 pipe (two lanes per clock and SM) the same
 // time for one lane as for 32, so this form is the faster one once there are
-// lines enough to fill warps on every SM (kPathWide).
-__global__ void __launch_bounds__(32) k_trace_path(const PathArgs A) {
+// lines enough to fill warps on every SM (kPathRuns).  BOTH: two runs a seed;
+// one run's constants then need no register (6001 lines, 600 points: 13.06
+// ms, 13.28 with the run picked by the grid row).
+template <bool BOTH>
+__global__ void __launch_bounds__(32) k_trace_path(const __grid_constant__ PathArgs A) {
     const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= A.n) return;
-    const PathRun R = A.run[blockIdx.y];
+    const PathRun& R = A.run[BOTH ? blockIdx.y : 0];
     double P[3] = {A.seeds[3 * s], A.seeds[3 * s + 1], A.seeds[3 * s + 2]};
     const double bound = (double)A.F.n[0];
     float* ox = A.ox + s * A.out_len;
@@ -262,7 +265,7 @@ __device__ __forceinline__ double bnorm_lanes(const PathField& F, const PathAxis
     return over_sqrt(a, __dadd_rn(__dadd_rn(pick3(q, base, 0), pick3(q, base, 1)), pick3(q, base, 2)));
 }
 
-__global__ void __launch_bounds__(32) k_trace_path_lanes(const PathArgs A) {
+__global__ void __launch_bounds__(32) k_trace_path_lanes(const __grid_constant__ PathArgs A) {
     const int lane = threadIdx.x, c = lane & 7, base = lane & 24;
     const long long s = (long long)blockIdx.x * 4 + (lane >> 3);
     const PathRun R = A.run[blockIdx.y];
@@ -297,17 +300,20 @@ __global__ void __launch_bounds__(32) k_trace_path_lanes(const PathArgs A) {
     }
 }
 
-// Lines up to which eight lanes share a line: the FP64 pipes of all SMs are
-// full from ~1000 lines on (both directions), and the time grows with the
-// lines from there (2000 points each way: 12.1 ms at 1000 lines), while one
-// lane to a line takes 42 ms for any number from 600 to 4000.
-constexpr long long kPathWide = 3000;
+// Runs (lines times directions) up to which eight lanes share one.  The FP64
+// pipes of all SMs are full from ~2000 runs on and the time grows with the
+// runs from there, while one lane to a run takes the same time for any number
+// up to a warp per pipe (~10,000 and, both ways, ~14,000): 600 points a run,
+// ms, eight lanes / one: 3000 runs 4.4 / 13.1, 6000 8.4 / 13.1, 8000 11.7 /
+// 13.1, 9000 12.6 / 13.1, 10,000 14.8 / 13.1, 12,000 16.8 / 13.1.
+constexpr long long kPathRuns = 9000;
 
 static cudaError_t launch_path(const PathArgs& A, int runs, cudaStream_t st) {
-    const bool wide = A.n * runs <= 2 * kPathWide;
+    const bool wide = A.n * runs <= kPathRuns;
     const dim3 grid((unsigned)(wide ? (A.n + 3) / 4 : (A.n + 31) / 32), (unsigned)runs);
     if (wide) k_trace_path_lanes<<<grid, 32, 0, st>>>(A);
-    else k_trace_path<<<grid, 32, 0, st>>>(A);
+    else if (runs == 1) k_trace_path<false><<<grid, 32, 0, st>>>(A);
+    else k_trace_path<true><<<grid, 32, 0, st>>>(A);
     return cudaGetLastError();
 }
 
