@@ -212,8 +212,9 @@ __device__ __forceinline__ double over_sqrt(double a, double s) {
     y = __fma_rn(y, e, y);
     const double d = __fma_rn(-g, g, s), h = nudge(y, -(1 << 20));
     const double r = __fma_rn(d, nudge(h, 1), g), r2 = __fma_rn(d, nudge(h, -1), g);
-    const double q = __dmul_rn(a, y), m = __fma_rn(-q, r, a);
-    const double u = __fma_rn(m, nudge(y, 1), q), u2 = __fma_rn(m, nudge(y, -1), q);
+    // (the remainder negated, so that a zero keeps its sign)
+    const double q = __dmul_rn(a, y), m = __fma_rn(q, r, -a);
+    const double u = __fma_rn(-m, nudge(y, 1), q), u2 = __fma_rn(-m, nudge(y, -1), q);
     // s in [2^-500, 2^500]: no step over- or underflows
     const int ex = (__double2hiint(s) >> 20) - 1023;
     const bool sure = (r == r2) & (u == u2) & (ex >= -500) & (ex <= 500);

@@ -688,11 +688,11 @@ struct Pending {
             L.len = L.len + d;
             if (tw_on) q = t * kInvPi;
         } else if (st == 2) {
-            if (tw_on) m = __fma_rn(-q, kRefPi, t);
+            if (tw_on) m = __fma_rn(q, kRefPi, -t);  // (negated: a zero keeps its sign)
         } else if (st == 3) {
             if (tw_on) {
-                u = __fma_rn(m, kInvPi * (1.0 + 0x1p-20), q);
-                v = __fma_rn(m, kInvPi * (1.0 - 0x1p-20), q);
+                u = __fma_rn(-m, kInvPi * (1.0 + 0x1p-20), q);
+                v = __fma_rn(-m, kInvPi * (1.0 - 0x1p-20), q);
             }
         }
     }
