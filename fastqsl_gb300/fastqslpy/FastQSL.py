@@ -83,8 +83,6 @@ def CookPseudoLine(x_end_arr, y_end_arr, z_end_arr, flag_end_arr,
     dev = bf.device
     n = int(bf.numel())
     lib = _lib.load()
-    # arrays of a kind as rows of one allocation (a zeroing or a copy is then
-    # one launch for all of them; each row is contiguous)
     cut = torch.empty((3, 4 * n), dtype=torch.float32, device=dev)
     bz0 = torch.empty((2, n), dtype=torch.float32, device=dev)
     count = torch.zeros(2, dtype=torch.int64, device=dev)
@@ -97,14 +95,24 @@ def CookPseudoLine(x_end_arr, y_end_arr, z_end_arr, flag_end_arr,
                "CookPseudoLine")
     k = int(count[0].item())
     m = 4 * k
-    cut_inp_x, cut_inp_y, cut_inp_z = cut[:, :m].clone(memory_format=torch.contiguous_format).unbind(0)
-    Bz0_start, Bz0_end = bz0[:, :k].clone(memory_format=torch.contiguous_format).unbind(0)
+    # every result an allocation of its own (one that a caller keeps holds no
+    # other, and each starts at the allocator's alignment), written by one
+    # launch per kind
+    new = lambda count, size, dtype=torch.float32: [torch.empty(size, dtype=dtype, device=dev)  # noqa: E731
+                                                    for _ in range(count)]
+    cut_inp, bz0_out = new(3, m), new(2, k)
+    torch._foreach_copy_(cut_inp + bz0_out, [c[:m] for c in cut] + [c[:k] for c in bz0])
+    zeros, flags = new(15, m), new(3, m, torch.int32)
+    torch._foreach_zero_(zeros)
+    torch._foreach_zero_(flags)
+    cut_inp_x, cut_inp_y, cut_inp_z = cut_inp
+    Bz0_start, Bz0_end = bz0_out
     (cut_start_x, cut_start_y, cut_start_z, cut_end_x, cut_end_y, cut_end_z,
      Bx_start_cut, By_start_cut, Bz_start_cut, Bx_end_cut, By_end_cut, Bz_end_cut,
-     Bx_inp_cut, By_inp_cut, Bz_inp_cut) = torch.zeros((15, m), dtype=torch.float32, device=dev).unbind(0)
+     Bx_inp_cut, By_inp_cut, Bz_inp_cut) = zeros
     line_len_cut = torch.zeros(m, dtype=torch.float64, device=dev)
     N_cut = _uint64(m, dev)
-    B_flag_cut, flag_cut_start, flag_cut_end = torch.zeros((3, m), dtype=torch.int32, device=dev).unbind(0)
+    B_flag_cut, flag_cut_start, flag_cut_end = flags
     return (cut_inp_x, cut_inp_y, cut_inp_z,
             cut_start_x, cut_start_y, cut_start_z, flag_cut_start,
             cut_end_x, cut_end_y, cut_end_z, flag_cut_end,
