@@ -1,11 +1,11 @@
 // One launch over many trace jobs: different fields (of one store type),
 // seed sets, integrators and tolerances.  Each job's lines occupy a
 // warp-aligned range [begin[j], begin[j] + n_j) of the launch's line space, so
-// no warp mixes two jobs; a thread finds its job by binary search over the
-// (small) begin table and traces one line with that job's settings, both ways,
-// lanes in lockstep.  Used for batched uneven solves (many
-// fields in one captured graph) and by the serving loop to merge the work of
-// concurrently admitted requests into one launch.
+// no warp mixes two jobs; a warp finds its job by binary search over the
+// (small) begin table and traces its lines with that job's settings, both
+// ways, lanes in lockstep.  Used for batched uneven solves (many fields in one
+// captured graph) and by the serving loop to merge the work of concurrently
+// admitted requests into one launch.
 #pragma once
 #include "qsl_trace.cuh"
 
@@ -24,10 +24,10 @@ struct BatchSlot {
 //
 // A job whose count comes from the device (n_dev) usually fills a small part
 // of its range, and the warps past it would start and exit.  When the whole
-// batch runs in one launch of its own, its lines go to all the job's warps: directions
-// to pairs of warps and up to four lanes per line, as in a launch of their
-// own (all after the main trace of two requests
-// of 17,000 seeds: 0.90 -> 0.75 ms).
+// batch runs in one launch with the GPU's idle lanes at its disposal, its
+// lines go to all the job's warps: directions to pairs of warps and up to four
+// lanes per line (all after the main trace of two requests of 17,000 seeds:
+// 0.90 -> 0.75 ms).
 template <class F>
 __device__ __forceinline__ BatchSlot batch_slot(const TraceJob<F>& J, long long n, long long g, long long begin,
                                                 long long room, bool whole) {

@@ -105,19 +105,20 @@ __device__ __forceinline__ float3 unit_and_grad_fd(const F& f, float3 p, float3 
 #pragma unroll
         for (int k = 0; k < 3; ++k) g[k] = oct_from(gj, base + 2 * k + 2);
         return oct_from(u, base);
-    }
-    const float3 b = sample<EXACT>(f, p, true);
+    } else {
+        const float3 b = sample<false>(f, p, true);
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        float3 lo = p, hi = p;
-        if (j == 0) { lo.x = lo.x - 0.001f; hi.x = hi.x + 0.001f; }
-        if (j == 1) { lo.y = lo.y - 0.001f; hi.y = hi.y + 0.001f; }
-        if (j == 2) { lo.z = lo.z - 0.001f; hi.z = hi.z + 0.001f; }
-        const float3 b1 = sample<EXACT>(f, lo, true);
-        const float3 b2 = sample<EXACT>(f, hi, true);
-        g[j] = 500.f * (b2 - b1);
+        for (int j = 0; j < 3; ++j) {
+            float3 lo = p, hi = p;
+            if (j == 0) { lo.x = lo.x - 0.001f; hi.x = hi.x + 0.001f; }
+            if (j == 1) { lo.y = lo.y - 0.001f; hi.y = hi.y + 0.001f; }
+            if (j == 2) { lo.z = lo.z - 0.001f; hi.z = hi.z + 0.001f; }
+            const float3 b1 = sample<false>(f, lo, true);
+            const float3 b2 = sample<false>(f, hi, true);
+            g[j] = 500.f * (b2 - b1);
+        }
+        return b;
     }
-    return b;
 }
 
 // Unit field and its exact gradient from one cell (fast arithmetic).
@@ -161,29 +162,29 @@ __device__ __forceinline__ Vec9 scott_rhs(const F& f, const Vec9& s, unsigned& n
     return {b, along(s.u, g), along(s.v, g)};
 }
 
-// Fehlberg step on the 9-vector; the error uses the position part only
-// (RKF45_Scott, TraceBlineScott.cu:256-290): its norm in exact arithmetic,
-// its square in fast arithmetic (the fast controller works with log2 of it).
-template <bool EXACT, int GRAD, class F>
+// Fehlberg step on the 9-vector in fast arithmetic; the error uses the position
+// part only (RKF45_Scott, TraceBlineScott.cu:256-290): its square (the fast
+// controller works with log2 of it).
+template <int GRAD, class F>
 __device__ __forceinline__ Vec9 scott_step(const F& f, const Vec9& s, float h, float& err, unsigned& ns) {
     using C = Fehlberg;
-    const Vec9 k1 = mul9(h, scott_rhs<EXACT, GRAD>(f, s, ns));
-    const Vec9 k2 = mul9(h, scott_rhs<EXACT, GRAD>(f, add9(s, mul9(C::a21, k1)), ns));
-    const Vec9 k3 = mul9(h, scott_rhs<EXACT, GRAD>(f, add9(s, add9(mul9(C::a31, k1), mul9(C::a32, k2))), ns));
-    const Vec9 k4 = mul9(h, scott_rhs<EXACT, GRAD>(
+    const Vec9 k1 = mul9(h, scott_rhs<false, GRAD>(f, s, ns));
+    const Vec9 k2 = mul9(h, scott_rhs<false, GRAD>(f, add9(s, mul9(C::a21, k1)), ns));
+    const Vec9 k3 = mul9(h, scott_rhs<false, GRAD>(f, add9(s, add9(mul9(C::a31, k1), mul9(C::a32, k2))), ns));
+    const Vec9 k4 = mul9(h, scott_rhs<false, GRAD>(
                                 f, add9(s, add9(add9(mul9(C::a41, k1), mul9(C::a42, k2)), mul9(C::a43, k3))), ns));
     const Vec9 k5 = mul9(
-        h, scott_rhs<EXACT, GRAD>(
+        h, scott_rhs<false, GRAD>(
                f, add9(s, add9(add9(add9(mul9(C::a51, k1), mul9(C::a52, k2)), mul9(C::a53, k3)), mul9(C::a54, k4))),
                ns));
     const Vec9 k6 = mul9(
-        h, scott_rhs<EXACT, GRAD>(
+        h, scott_rhs<false, GRAD>(
                f,
                add9(s, add9(add9(add9(add9(mul9(C::a61, k1), mul9(C::a62, k2)), mul9(C::a63, k3)), mul9(C::a64, k4)),
                             mul9(C::a65, k5))),
                ns));
     const float3 e = (((C::e1 * k1.p + C::e3 * k3.p) + C::e4 * k4.p) + C::e5 * k5.p) + C::e6 * k6.p;
-    err = EXACT ? norm(e) : fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z));
+    err = fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z));
     return add9(s, add9(add9(add9(add9(mul9(C::b1, k1), mul9(C::b3, k3)), mul9(C::b4, k4)), mul9(C::b5, k5)),
                         mul9(C::b6, k6)));
 }
@@ -240,7 +241,7 @@ __device__ __forceinline__ Vec9 scott_step_rolled(const F& f, const Vec9& s, flo
 
 // The exact Fehlberg step with rolled stages: the same products and sums in
 // the same order as scott_step (each stage's k adds its term to the sums
-// still to come, from the left).
+// still to come, from the left); the error is the norm.
 template <int GRAD, class F>
 __device__ __forceinline__ Vec9 scott_step_exact(const F& f, const Vec9& s, float h, float& err, unsigned& ns) {
     const Vec9 zero = {v3(0.f, 0.f, 0.f), v3(0.f, 0.f, 0.f), v3(0.f, 0.f, 0.f)};
@@ -355,7 +356,7 @@ __device__ void scott_line(const F& f, const ScottJob<F>& J, long long i, float 
             // analytic gradient's one fetch keeps the unrolled step (3.4 ms
             // against 3.8 rolled)
             if constexpr (EXACT) b = scott_step_exact<GRAD>(f, a, h * (float)sgn, err, ns);
-            else if constexpr (GRAD == GRAD_ANALYTIC) b = scott_step<EXACT, GRAD>(f, a, h * (float)sgn, err, ns);
+            else if constexpr (GRAD == GRAD_ANALYTIC) b = scott_step<GRAD>(f, a, h * (float)sgn, err, ns);
             else b = scott_step_rolled<GRAD>(f, a, h * (float)sgn, err, ns);
             if (EXACT) {
                 const float scale = step_scale_exact(tol / err);

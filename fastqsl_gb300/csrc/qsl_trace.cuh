@@ -212,15 +212,9 @@ __device__ __forceinline__ float3 step_rkf45_fast_rolled(const F& f, float3 p, f
     return f3(scal(h, sol));
 }
 
-// The exact Fehlberg step: k = h b per stage, every product and sum rounded on
-// its own in the reference's order (sums from the left; a stage's input is
-// p plus its whole sum).  The stages are rolled as above: each stage's k adds
-// its term to the sums still to come, which is that order.  (Unrolled, the
-// exact samples do not fit the instruction cache: drop-in planes 18-35 %
-// slower.)
-// aside(st) runs at the start of stage st: work whose results are not needed
-// in the step (Lane's pending sums), placed where the stage's sample hides
-// its latency.
+// aside(st) runs at the start of stage st of an exact step: work whose results
+// are not needed in the step (Lane's pending sums), placed where the stage's
+// sample hides its latency.  Without any:
 struct Nothing {
     __device__ __forceinline__ void operator()(int) const {}
     template <class F>
@@ -239,6 +233,12 @@ __device__ __forceinline__ float3 stage_exact(const F& f, float3 p, int st, A& a
     aside.field(f, st, cell, w, raw);
     return unit_exact(raw);
 }
+// The exact Fehlberg step: k = h b per stage, every product and sum rounded on
+// its own in the reference's order (sums from the left; a stage's input is
+// p plus its whole sum).  The stages are rolled as above: each stage's k adds
+// its term to the sums still to come, which is that order.  (Unrolled, the
+// exact samples do not fit the instruction cache: drop-in planes 18-35 %
+// slower.)
 template <class F, class A>
 __device__ __forceinline__ float3 step_rkf45_exact(const F& f, float3 p, float h, float& err, unsigned& ns, A& aside) {
     const float3 zero = v3(0.f, 0.f, 0.f);
@@ -270,8 +270,6 @@ __device__ __forceinline__ float3 step_rkf45(const F& f, float3 p, float h, floa
     else return step_rkf45_fast(f, p, h, err, ns, b_raw);
 }
 
-// Classic RK4 on b (RK4, TraceBlineAdaptive.cu:259-267); returns the
-// increment.  The 1/6 factor is formed as (1./6.)*h in double and narrowed.
 // (float)((1. / 6.) * (double)h) without the FP64 pipe: h times the double
 // 1/6 held as two floats.
 __device__ __forceinline__ float sixth_exact(float h) {
@@ -283,11 +281,14 @@ __device__ __forceinline__ float sixth_exact(float h) {
     return sure ? r : (float)(y * (double)h);
 }
 
+// Classic RK4 on b (RK4, TraceBlineAdaptive.cu:259-267); returns the
+// increment.  Exact arithmetic: the 1/6 factor as (1./6.)*h rounded once, and
+// the stages rolled (one sample in the loop body; the same operations in the
+// same order).
 template <bool EXACT, class F, class A>
 __device__ __forceinline__ float3 step_rk4(const F& f, float3 p, float h, unsigned& ns, float3* b_raw, A& aside) {
+    ns += 4;
     if constexpr (EXACT) {
-        // the stages rolled (one sample in the loop body): the same
-        // operations in the same order
         float3 q = p, sum = v3(0.f, 0.f, 0.f);
 #pragma unroll 1
         for (int st = 0; st < 4; ++st) {
@@ -297,15 +298,14 @@ __device__ __forceinline__ float3 step_rk4(const F& f, float3 p, float h, unsign
             q = p + (st < 2 ? 0.5f * hk : hk);
             sum = st == 0 ? k : (st < 3 ? sum + 2.f * k : sum + k);
         }
-        ns += 4;
         return sixth_exact(h) * sum;
+    } else {
+        const float3 k1 = b_raw ? sample_unit_raw(f, p, *b_raw) : sample<false>(f, p, true);
+        const float3 k2 = sample<false>(f, p + (h * k1) / 2.f, true);
+        const float3 k3 = sample<false>(f, p + (h * k2) / 2.f, true);
+        const float3 k4 = sample<false>(f, p + h * k3, true);
+        return h * (1.f / 6.f) * (((k1 + 2.f * k2) + 2.f * k3) + k4);
     }
-    const float3 k1 = b_raw ? sample_unit_raw(f, p, *b_raw) : sample<EXACT>(f, p, true);
-    const float3 k2 = sample<EXACT>(f, p + (h * k1) / 2.f, true);
-    const float3 k3 = sample<EXACT>(f, p + (h * k2) / 2.f, true);
-    const float3 k4 = sample<EXACT>(f, p + h * k3, true);
-    ns += 4;
-    return h * (1.f / 6.f) * (((k1 + 2.f * k2) + 2.f * k3) + k4);
 }
 
 // RK4 in the face-normal coordinate, dx/dq = b / b_d over dq = h
@@ -975,9 +975,7 @@ __device__ __forceinline__ void lane_turn(const TraceJob<F>& J, Lane<EXACT>& L, 
 // What a finished direction leaves behind until its warp's other lanes are
 // done (lane_foot and the outputs then run once for the whole warp): an
 // array per lane, one row per direction.  Indexed by the direction it lives
-// in local memory, which the stepping loop does not touch (as 4.6 KB of
-// shared memory per block it took 4 % off the L1-bound Q cube, 113.4 ->
-// 117.7 ms).
+// in local memory, which the stepping loop does not touch.
 template <bool EXACT>
 struct Stash {
     float p[3], q[3];
