@@ -983,7 +983,11 @@ struct Stash {
     float lc;
     typename Lane<EXACT>::len_t len;
     double tw;
-    long long line;  // trace_queue: the lane's line (of S[0])
+};
+// (trace_queue's rows; kept apart so that other kernels' frames stay small)
+template <bool EXACT>
+struct QueueStash : Stash<EXACT> {
+    long long line;  // the lane's line (of S[0])
 };
 template <bool EXACT, bool TWIST>
 __device__ __forceinline__ void stash_put(Stash<EXACT>& S, const Lane<EXACT>& L) {
@@ -1017,8 +1021,8 @@ __device__ __forceinline__ void pair_sync() {
 
 // The end of a warp's lines, for all its lanes at once: the footpoints and
 // samples of B of the directions in S and the outputs.
-template <bool EXACT, bool TWIST, class F>
-__device__ __forceinline__ unsigned lines_finish(const F& f, const TraceJob<F>& J, const Stash<EXACT>* S, long long i,
+template <bool EXACT, bool TWIST, class F, class Rows>
+__device__ __forceinline__ unsigned lines_finish(const F& f, const TraceJob<F>& J, const Rows* S, long long i,
                                          bool valid, bool split, float3 nrm, bool tw_on) {
     Lane<EXACT> L;
     unsigned ns = 0;
@@ -1126,31 +1130,43 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 //
 // When it refills: a partial refill costs the coherence of a warp of
 // neighbours and does the ends for a part of its lanes, so it has to be
-// worth that.  kRefillLanes idle lanes; kRefillIdle looks, kRefillSteps trial
-// steps apart, summed over the idle lanes (64 steps of the whole warp); and
-// idle lane steps of a 1 / (1 + kRefillShare) part of all since the last
-// refill.  200,000 lines, ms, one refill per line as it ends / none before the
-// last line of 32 / this: a field whose lines are 3 % ropes of ten times the
-// mean length, bricks 8.0 / 9.8 / 6.7, float4 7.6 / 11.2 / 7.3, drop-in RKF45
-// 480 / 146 / 130; seeds anywhere in a charge field's volume 3.6 / 3.5 / 3.4,
-// 4.9 / 5.1 / 4.7, 37 / 11.5 / 9.3; its bottom plane in random order 1.9 /
-// 2.2 / 1.65, row by row 1.7 / 1.43 / 1.45.  What it costs: planes that are
-// coherent and even, 258 x 258 x 32 seeds on bricks in tile order 13.4 -> 14.0
-// (none -> this; 12.4 static), drop-in twist on 201 x 203 x 4 seeds 2.59 ->
-// 2.62.  Without the second and third rule (16 idle lanes alone) those two
-// were 14.6 and 2.67.
+// worth that.  A warp whose seeds are neighbours (`neighbours`: a 1 /
+// kNeighbours of the box's edges summed is 2-3 cells of a 64^3 box) waits for
+// its last line: their lengths are alike, and what is left of such a warp
+// costs little.  Others refill at kRefillLanes idle lanes; kRefillIdle looks,
+// kRefillSteps trial steps apart, summed over the idle lanes (64 steps of the
+// whole warp); and idle lane steps of a 1 / (1 + kRefillShare) part of all
+// since the last refill.  200,000 lines, ms, one refill per line as it ends /
+// none before the last line of 32 / this: a field whose lines are 3 % ropes of
+// ten times the mean length, bricks 8.0 / 9.8 / 6.8, float4 7.6 / 11.2 / 7.3,
+// drop-in RKF45 480 / 146 / 137; seeds anywhere in a charge field's volume
+// 3.6 / 3.5 / 3.4, 4.9 / 5.1 / 4.7, 37 / 11.5 / 9.3; its bottom plane in
+// random order 1.9 / 2.2 / 1.65.  Coherent, even planes (none / refills
+// whatever the seeds / this): 258 x 258 x 32 seeds on bricks in tile order
+// 13.77 / 13.85 / 13.80, drop-in twist on 201 x 203 x 4 seeds 3.05 / 3.15 /
+// 3.07 and 2.83 / 2.92 / 2.84.
 constexpr int kRefillSteps = 8;
 constexpr int kRefillLanes = 16;
 constexpr unsigned kRefillIdle = 256;
 constexpr unsigned kRefillShare = 2;
+constexpr float kNeighbours = 64.f;
+// Whether a warp's seeds are neighbours: all but a quarter of them within
+// `apart`, per axis, of the lane before.
+__device__ __forceinline__ bool neighbours(float3 p, bool active, float apart) {
+    const float3 d = p - v3(__shfl_up_sync(0xffffffffu, p.x, 1), __shfl_up_sync(0xffffffffu, p.y, 1),
+                            __shfl_up_sync(0xffffffffu, p.z, 1));
+    const bool far = active & (fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z)) > apart);
+    return __popc(__ballot_sync(0xffffffffu, far)) <= 8;
+}
 template <bool EXACT, bool TWIST, class F, class N, class SL, class TC, class NR>
 __device__ __forceinline__ void trace_queue(const F& f, const TraceJob<F>& J, const N& n_of,
                                             const LenLimit<EXACT>& limit, const SL& s_len_of, const TC& tol_coef_of,
                                             const NR& nrm_of, bool tw_on, unsigned& ns) {
     Lane<EXACT> L;
-    Stash<EXACT> S[2];
+    QueueStash<EXACT> S[2];
     bool active = false, ended = false;
-    bool drained = false;  // (warp-uniform) the counter is past the last line
+    // (warp-uniform) the counter is past the last line; the warp's seeds are neighbours
+    bool drained = false, together = false;
     while (true) {
         if (__any_sync(0xffffffffu, ended)) {
             ns += lines_finish<EXACT, TWIST>(f, J, S, S[0].line, ended, false, nrm_of(), tw_on);
@@ -1163,6 +1179,7 @@ __device__ __forceinline__ void trace_queue(const F& f, const TraceJob<F>& J, co
             }
         }
         unsigned want = __ballot_sync(0xffffffffu, !active);
+        const bool fresh = want == 0xffffffffu;
         while (want != 0u && !drained) {
             // no more than the idle lanes: what a warp held back for later
             // (a chunk of 256) waited while others had nothing left
@@ -1182,10 +1199,12 @@ __device__ __forceinline__ void trace_queue(const F& f, const TraceJob<F>& J, co
             want = __ballot_sync(0xffffffffu, !active);
         }
         if (!__any_sync(0xffffffffu, active)) break;
+        if (fresh) together = neighbours(L.p, active, (float)len_scale(f) * (1.f / kNeighbours));
+        const bool wait = drained | together;
         int idle;
         unsigned busy_steps = 0, idle_steps = 0;
         do {
-            for (int k = drained ? 0x7fffffff : kRefillSteps; active && k > 0; --k) {
+            for (int k = wait ? 0x7fffffff : kRefillSteps; active && k > 0; --k) {
                 if (!lane_step<EXACT, TWIST>(f, J, L, limit, tw_on, ns)) continue;
                 stash_put<EXACT, TWIST>(S[L.dsign >> 31], L);
                 if (L.dsign == 0) {
@@ -1198,7 +1217,7 @@ __device__ __forceinline__ void trace_queue(const F& f, const TraceJob<F>& J, co
             idle = __popc(__ballot_sync(0xffffffffu, !active));
             idle_steps += idle;
             busy_steps += 32 - idle;
-        } while (idle < 32 && (drained || idle < kRefillLanes || idle_steps < kRefillIdle ||
+        } while (idle < 32 && (wait || idle < kRefillLanes || idle_steps < kRefillIdle ||
                                kRefillShare * idle_steps < busy_steps));
     }
 }
@@ -1229,14 +1248,30 @@ __host__ __device__ __forceinline__ LaunchShape launch_shape(long long n, long l
     return {split, split ? spread_of(n, warps) : 1};
 }
 
+// A queue launch with a lane for every line and more than three quarters of its
+// lanes in use takes its warps' lines from the counter, in the order in which
+// the warps come: a block's four warps then hold lines from four places, where
+// by index they hold neighbours, which are long together.  Below that, lines by
+// index fill whole blocks, which lie evenly over the SMs.  Drop-ins on 152 x 4
+// blocks, ms, from the counter / by index: 98 % of the lanes 0.87 / 0.89 and
+// 1.07 / 1.10 (stretched), 1.77 / 1.79 and 1.73 / 1.75 (RKF45), 96 % 0.92 /
+// 0.96 and 1.04 / 1.13, 80 % 1.74 / 1.71 and 1.67 / 1.71, 66 % 1.66 / 1.58 and
+// 1.66 / 1.59, 51 % 1.61 / 1.44 and 1.58 / 1.45.
+__host__ __device__ __forceinline__ bool scattered(long long n, long long warps) { return 4 * n > 3 * 32 * warps; }
+// (out of line: inlined, RK4 drop-ins, which never take it, 3.46 -> 3.50 ms)
+static __device__ __noinline__ unsigned queue_turn(unsigned long long* queue) {
+    unsigned turn = 0;
+    if ((threadIdx.x & 31) == 0) turn = (unsigned)atomicAdd(queue, 1ull);
+    return __shfl_sync(0xffffffffu, turn, 0);
+}
+
 // The tracer kernel.  QUEUE = true and more lines than the grid has lanes:
 // warps take lines from the device counter J.queue (trace_queue).  Else every
 // warp takes 32 lines at a time and traces them in lockstep, line = global
-// thread index + k * total threads; a launch whose grid has two threads per
-// line splits the directions over warp pairs (trace_lines).  (A queue launch
-// with a lane for every line: a plane of 250 x 300 seeds on a stretched grid
-// 1.24 ms from the counter, 1.19 so.)  Lines are visited in J.order when it
-// is set.  TWIST compiles the twist integral in; it runs when the runtime
+// thread index + k * total threads (the warp's index from the counter where
+// `scattered` says so); a launch whose grid has two threads per line splits
+// the directions over warp pairs (trace_lines).  Lines are visited in J.order
+// when it is set.  TWIST compiles the twist integral in; it runs when the runtime
 // flag is set.
 template <bool EXACT, bool TWIST, bool QUEUE, class F>
 __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
@@ -1285,14 +1320,16 @@ __device__ __forceinline__ void trace_kernel_body(const TraceJob<F>& J) {
     unsigned ns = 0;
     const int lane_id = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (blockDim.x / 32);
-    const LaunchShape shape = launch_shape(n_of(), warps);
-    const bool split = shape.split;
-    const int spread = shape.spread;
+    // (launch_shape's values: a struct of them spills in the stretched kernels)
+    const bool split = splits(n_of(), warps);
+    const int spread = split ? spread_of(n_of(), warps) : 1;
     const int lines = 32 / spread;  // of a warp
     if (QUEUE && n_of() > 32 * warps) {
         trace_queue<EXACT, TWIST>(f, J, n_of, limit, s_len_of, tol_coef_of, nrm_of, tw_on, ns);
     } else {
-        long long line = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+        long long line = QUEUE && scattered(n_of(), warps)
+                             ? (long long)queue_turn(J.queue)
+                             : (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
         for (line = (split ? line >> 1 : line) * lines; line < n_of(); line += warps * lines / (split ? 2 : 1)) {
             const long long slot = line + lane_id / spread;
             const bool valid = lane_id % spread == 0 && slot < n_of();

@@ -92,3 +92,20 @@ def test_samples_and_order_do_not_depend_on_refills(ropes):
         runs.append((int(count.item()), out["LineLen"].cpu().numpy(), out["end_x"].cpu().numpy()))
     assert runs[0][0] == runs[1][0]
     assert all(np.array_equal(x, y) for x, y in zip(runs[0][1:], runs[1][1:]))
+
+
+@pytest.mark.parametrize("layout", ["soa", "h4b"])
+def test_neighbours_and_others_in_one_launch(ropes, layout):
+    """Warps whose seeds are neighbours (rows of a plane) wait for their last
+    line, others refill; a warp may change from one to the other."""
+    from fastqsl_gb300 import api
+    field, seeds = ropes
+    k = torch.arange(N // 2, device="cuda", dtype=torch.float32)
+    rows = [0.25 * (k % 600) + 2.0, 0.9 * (k // 600) + 2.0, torch.full_like(k, 3.0)]
+    s = [torch.cat([r, a[:N // 2]]).contiguous() for r, a in zip(rows, seeds)]
+    store = api.FieldStore(*field, layout=layout)
+    prm = P.reference_rkf45() if layout == "soa" else P.absolute_rkf45(tol=1e-4)
+    a, b = (api.trace(store, *s, prm, s_len=0.25, schedule=q, status=True) for q in ("static", "queue"))
+    for name, v in a.items():
+        assert v is None or np.array_equal(v.cpu().numpy(), b[name].cpu().numpy(),
+                                           equal_nan=v.is_floating_point()), name
