@@ -596,6 +596,10 @@ def _hybrid_impl(self, field, xs, ys, zs, params, s_len, tol_coef, scott_params,
 QMapPlan._hybrid = _hybrid_impl
 
 
+# resident blocks per SM of the batched kernels at occupancy 0
+BATCH_BLOCKS_PER_SM = 6
+
+
 class PlaneQBatch:
     """Q maps of many plane jobs as one native batch (qsl_qmap_batch_*): the
     seed grids, tile orders, job tables, batched traces and the batched Q

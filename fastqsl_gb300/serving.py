@@ -17,9 +17,10 @@ sub-box) and an RKF45 tolerance.  The scheduler loop:
   CUDA streams, so a batch starts while earlier ones are still on the GPU and
   their work overlaps on the device.  Smaller classes run on higher-priority
   streams: their blocks are dispatched ahead of a large batch's remaining
-  blocks, and larger classes keep at most `big_blocks_per_sm` of the 8
-  resident block slots per SM, so a small request finds free slots at once
-  instead of waiting for a large batch's blocks to retire;
+  blocks, and larger classes' batches that run whole (chunk_lines=0) keep to
+  `big_blocks_per_sm` of the batched kernels' 6 resident blocks per SM, so a
+  small request finds free slots at once instead of waiting for a large
+  batch's blocks to retire;
 * runs the main trace of larger classes' batches as windows of
   `chunk_lines` lines (qsl_batch_run_window), at most `max_chunks` windows
   on the device at a time and `chunks_when_interactive` while a batch of the
@@ -30,8 +31,8 @@ sub-box) and an RKF45 tolerance.  The scheduler loop:
 Nothing in the loop synchronises the device: allocations come from the
 caching allocator on the batch's stream, the job table is copied
 asynchronously from pinned memory, completion is polled.  A request's result
-does not depend on what it was batched with (each line is traced by one
-thread with its job's settings; tests check alone == in the mix bit for bit).
+does not depend on what it was batched with (each line is traced on its own
+with its job's settings; tests check alone == in the mix bit for bit).
 """
 from __future__ import annotations
 
@@ -160,7 +161,7 @@ class QServer:
     CLASSES = ((1.5e5, 2, 12), (1.2e6, 2, 3), (float("inf"), 1, 3))
 
     def __init__(self, fields, hbm_budget=16 << 30, streams=2, max_batch=None, s_len=0.25, h_min=1e-3, h_max=1.0,
-                 tile=(8, 8), device="cuda", classes=None, big_blocks_per_sm=6, chunk_lines=1 << 17, max_chunks=4,
+                 tile=(8, 8), device="cuda", classes=None, big_blocks_per_sm=5, chunk_lines=1 << 17, max_chunks=4,
                  chunks_when_interactive=3, window_streams=2, window_blocks_per_sm=0, window_order="srpt"):
         self.fields = dict(fields)
         self.budget = int(hbm_budget)
@@ -183,9 +184,12 @@ class QServer:
         self.s_len, self.h_min, self.h_max = s_len, h_min, h_max
         self.tile = tile
         # batches of all but the smallest class, where they run whole, keep at
-        # most this many blocks per SM (6 are resident at the batched kernels'
-        # default budget), each looping over its lines; fewer leave slots in
-        # which the smallest requests' blocks start at once (0 = no cap)
+        # most this many blocks per SM, each looping over its lines, of the
+        # api.BATCH_BLOCKS_PER_SM that are resident: the smallest requests'
+        # blocks start at once in the rest (0 = no cap).  10^4-4x10^6 seeds,
+        # whole batches, p99 in ms of the smallest class at 63 and 101
+        # requests/s and M Q-px/s saturated: 6 blocks 53, 128 and 90; 5: 45, 98
+        # and 90; 4: 45, 99 and 90; 3: 62, 83 and 88
         self.big_blocks_per_sm = int(big_blocks_per_sm)
         # main traces of classes > 0 run as windows of chunk_lines lines (a
         # multiple of 32; 0 = one launch per batch)
