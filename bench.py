@@ -867,8 +867,8 @@ def main():
                                  "frac": flops / k_s / 1e12 / fp32_peak, "peak_kind": "nominal",
                                  "sm_count": res["sm_count"]}
     line["roofline"]["limiter"] = ("SM issue, the FMA pipe and the L1 data pipe together (ncu on 32 mid-cube "
-                                   "planes: issue active ~74 %, FMA pipe ~64 % of its cycles, L1 LSU wavefronts "
-                                   "~76 % of peak)")
+                                   "planes at 6 blocks per SM: issue active ~72 %, FMA pipe ~65 % of its cycles, "
+                                   "L1 LSU wavefronts ~77 % of peak)")
     # launches per step: main trace, qcalc, flag_count, tile_scan, cook_write,
     # pseudo trace, qcut with the merge (+ 2 memsets of the queue counters)
     line["gpu_launches"] = 7 * args.steps
